@@ -120,6 +120,7 @@ Engine::~Engine() {
     fr(turns_); fr(bigram_);
     each_linear([&](LinearW& w) { fr(w.slabs); fr(w.tc); fr(w.scales); fr(w.codes); fr(w.kq_data); fr(w.kq_tile_type); });
     free_listed();
+    free_wide();
     free_listed_cache();
     fr(hsel_); fr(st_tokens_); fr(st_pos_); fr(st_seq_); fr(st_want_); fr(st_next_); fr(seq_iota_);
     if (st_pin_) cudaFreeHost(st_pin_);
@@ -1078,6 +1079,37 @@ int Engine::enqueue_linear(const LinearW& L, int M, const float* x, int ldx, int
     return HM_OK;
 }
 
+AttnArgs Engine::attn_args(int l, int M, const float* q, const int32_t* row_pos, const int32_t* row_seq) const {
+    AttnArgs at{};
+    at.q = q;
+    at.k_pool = k_pool_[l];
+    at.v_pool = v_pool_[l];
+    at.page_table = page_table_;
+    at.row_seq = row_seq;
+    at.row_pos = row_pos;
+    at.kv_len = nullptr;
+    at.max_pages = max_pages_;
+    at.page_tokens = page_tokens_;
+    at.heads = heads_;
+    at.kv_heads = kvh_;
+    at.hd = hd_;
+    // fewer splits when the rows alone fill the SMs: about two CTAs per SM on the cluster path (caches
+    // of up to 1024 tokens), the kernel's cost model on the long-context path
+    at.nsplit = std::min(att_nsplit_, att_cluster_ ? std::max(1, (2 * sm_count_ + M * kvh_ - 1) / (M * kvh_)) : attn_pick_nsplit(M, kvh_, max_pages_, sm_count_, kv_bf16_));
+    at.cluster = att_cluster_ ? 1 : 0;
+    at.stream_pages = 1;
+    // decode passes: one row per sequence (prefill chunks write several positions of one sequence); launches of at most two
+    // CTAs per SM are latency-bound and keep all their pages resident, larger ones keep their shared memory small
+    at.early_pages = row_seq == nullptr ? ((long)M * kvh_ * at.nsplit <= 2L * sm_count_ ? 2 : 1) : 0;
+    at.err_flag = err_flag_;
+    at.scale = (float)(1.0 / std::sqrt((double)hd_));  // src/hf/emitter.rs:719
+    at.out = attn_;
+    at.part_acc = att_acc_;
+    at.part_ml = att_ml_;
+    at.tickets = att_tickets_;
+    return at;
+}
+
 int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_pos, const int32_t* row_seq, int lm_row0, int lm_rows, bool advance, uint32_t* next_dev, uint32_t* feed_dev,
                          int32_t* pos_dev, uint32_t* hist_dev, int* launches) {
     (void)advance;
@@ -1168,24 +1200,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
             if (ce != cudaSuccess) return cuda_fail(ce, "post_qkv");
             ++*launches;
         }
-        AttnArgs at{};
-        at.q = q_;
-        at.k_pool = k_pool_[l];
-        at.v_pool = v_pool_[l];
-        at.page_table = page_table_;
-        at.row_seq = row_seq;
-        at.row_pos = row_pos;
-        at.kv_len = nullptr;
-        at.max_pages = max_pages_;
-        at.page_tokens = page_tokens_;
-        at.heads = heads_;
-        at.kv_heads = kvh_;
-        at.hd = hd_;
-        // fewer splits when the rows alone fill the SMs: about two CTAs per SM on the cluster path (caches
-        // of up to 1024 tokens), the kernel's cost model on the long-context path
-        at.nsplit = std::min(att_nsplit_, att_cluster_ ? std::max(1, (2 * sm_count_ + M * kvh_ - 1) / (M * kvh_)) : attn_pick_nsplit(M, kvh_, max_pages_, sm_count_, kv_bf16_));
-        at.cluster = att_cluster_ ? 1 : 0;
-        at.stream_pages = 1;
+        AttnArgs at = attn_args(l, M, q_, row_pos, row_seq);
         if (direct_pack) {
             at.xp_out = xpack_attn_;
             at.xp_mpad = tc_mpad(M);
@@ -1193,15 +1208,6 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
 #ifdef HM_PHASE_TRACE
         if (gemv_trace_ && *launches < 512) at.trace = gemv_trace_ + (size_t)*launches * 16;
 #endif
-        // decode passes: one row per sequence (prefill chunks write several positions of one sequence); launches of at most two
-        // CTAs per SM are latency-bound and keep all their pages resident, larger ones keep their shared memory small
-        at.early_pages = row_seq == nullptr ? ((long)M * kvh_ * at.nsplit <= 2L * sm_count_ ? 2 : 1) : 0;
-        at.err_flag = err_flag_;
-        at.scale = (float)(1.0 / std::sqrt((double)hd_));  // src/hf/emitter.rs:719
-        at.out = attn_;
-        at.part_acc = att_acc_;
-        at.part_ml = att_ml_;
-        at.tickets = att_tickets_;
         if (pf) {
             at.pf_ptr = w.gu.slabs;
             at.pf_bytes = w.gu.bytes();
@@ -1263,7 +1269,6 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
         if (rc) return rc;
     }
     if (lm_rows > 0) {
-        const int nslabs = (V_ + SLAB - 1) / SLAB;
         const float* x = h_ + (size_t)lm_row0 * H_;
         if (lm_pick_) {  // rows of a mixed batch whose logits are wanted
             ce = launch_gather_rows(h_, lm_pick_, lm_rows, H_, hsel_, stream_, pdl_);
@@ -1271,41 +1276,52 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
             ++*launches;
             x = hsel_;
         }
-        float* const lg = logits_ + lm_dst_row_ * V_;
-        const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows);
-        const bool slab_argmax = lm_head_.kind == HM_BF16;  // per-block argmax partials from the projection's epilogue
-        const bool fold_argmax = slab_argmax && !lm_tall;    // the streaming kernel's last epilogue also produces the greedy token
-        lm_folds_argmax_ = fold_argmax;
-        if (spec_.listed()) {
-            if (want(PC_LM_HEAD) && spec_.sandwich) {
-                rc = enqueue_sandwich_logits(x, lm_rows, final_norm_fits(M, lm_rows), (lm_out_ && fold_argmax) ? lm_out_ : lg, ArgmaxFold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1}, launches);
-                if (rc) return rc;
-            } else if (want(PC_LM_HEAD)) {
-                rc = enqueue_listed_logits(x, lm_rows, (lm_out_ && fold_argmax) ? lm_out_ : lg, ArgmaxFold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1}, launches);
-                if (rc) return rc;
-            }
-        } else if (want(PC_LM_HEAD) && lm_tall && fused && lm_row0 == 0 && lm_rows == M && !lm_pick_) {
-            TcFuse f;
-            f.ss_in = ss_h_;
-            f.ss_parts = H_ / 128;
-            rc = enqueue_linear_tc(lm_head_, lm_rows, x, H_, nullptr, EPI_LOGITS, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, launches, xpack_h_, nullptr, &f);
-            if (rc) return rc;
-        } else if (want(PC_LM_HEAD) && lm_tall) {
-            rc = enqueue_linear_tc(lm_head_, lm_rows, x, H_, final_norm_, EPI_LOGITS, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, launches);
+        return enqueue_logits(x, lm_rows, final_norm_fits(M, lm_rows), fused && lm_row0 == 0 && lm_rows == M && !lm_pick_, next_dev, feed_dev, pos_dev, hist_dev, launches);
+    }
+    return HM_OK;
+}
+
+// Final norm, LM head and argmax of up to scratch_rows_ rows x.  whole_pass: they are all rows of the pass enqueued last; packed: and its
+// last projection left them packed in xpack_h_ with their sums of squares.
+int Engine::enqueue_logits(const float* x, int lm_rows, bool whole_pass, bool packed, uint32_t* next_dev, uint32_t* feed_dev, int32_t* pos_dev, uint32_t* hist_dev, int* launches) {
+    auto want = [&](int cls) { return only_class_ < 0 || only_class_ == cls; };
+    cudaError_t ce = cudaSuccess;
+    int rc;
+    const int nslabs = (V_ + SLAB - 1) / SLAB;
+    float* const lg = logits_ + lm_dst_row_ * V_;
+    const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows);
+    const bool slab_argmax = lm_head_.kind == HM_BF16;  // per-block argmax partials from the projection's epilogue
+    const bool fold_argmax = slab_argmax && !lm_tall;    // the streaming kernel's last epilogue also produces the greedy token
+    lm_folds_argmax_ = fold_argmax;
+    if (spec_.listed()) {
+        if (want(PC_LM_HEAD) && spec_.sandwich) {
+            rc = enqueue_sandwich_logits(x, lm_rows, whole_pass, (lm_out_ && fold_argmax) ? lm_out_ : lg, ArgmaxFold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1}, launches);
             if (rc) return rc;
         } else if (want(PC_LM_HEAD)) {
-            const ArgmaxFold fold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1};
-            float* lm_dst = (lm_out_ && fold_argmax) ? lm_out_ : logits_;
-            rc = slab_argmax ? enqueue_linear(lm_head_, lm_rows, x, H_, PRO_RMSNORM, final_norm_, EPI_LOGITS, lm_dst, V_, nullptr, nullptr, -1, nullptr, nullptr, amax_val_, amax_idx_, launches, &fold)
-                             : enqueue_linear(lm_head_, lm_rows, x, H_, PRO_RMSNORM, final_norm_, EPI_STORE, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, nullptr, nullptr, launches);
+            rc = enqueue_listed_logits(x, lm_rows, (lm_out_ && fold_argmax) ? lm_out_ : lg, ArgmaxFold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1}, launches);
             if (rc) return rc;
         }
-        if (want(PC_SAMPLE) && !fold_argmax) {
-            ce = slab_argmax ? launch_argmax_finish(amax_val_, amax_idx_, nslabs, lm_rows, next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1, stream_, pdl_)
-                             : launch_argmax_finish(lg, nullptr, V_, lm_rows, next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1, stream_, pdl_);
-            if (ce != cudaSuccess) return cuda_fail(ce, "argmax_finish");
-            ++*launches;
-        }
+    } else if (want(PC_LM_HEAD) && lm_tall && packed) {
+        TcFuse f;
+        f.ss_in = ss_h_;
+        f.ss_parts = H_ / 128;
+        rc = enqueue_linear_tc(lm_head_, lm_rows, x, H_, nullptr, EPI_LOGITS, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, launches, xpack_h_, nullptr, &f);
+        if (rc) return rc;
+    } else if (want(PC_LM_HEAD) && lm_tall) {
+        rc = enqueue_linear_tc(lm_head_, lm_rows, x, H_, final_norm_, EPI_LOGITS, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, launches);
+        if (rc) return rc;
+    } else if (want(PC_LM_HEAD)) {
+        const ArgmaxFold fold{next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1};
+        float* lm_dst = (lm_out_ && fold_argmax) ? lm_out_ : logits_;
+        rc = slab_argmax ? enqueue_linear(lm_head_, lm_rows, x, H_, PRO_RMSNORM, final_norm_, EPI_LOGITS, lm_dst, V_, nullptr, nullptr, -1, nullptr, nullptr, amax_val_, amax_idx_, launches, &fold)
+                         : enqueue_linear(lm_head_, lm_rows, x, H_, PRO_RMSNORM, final_norm_, EPI_STORE, logits_, V_, nullptr, nullptr, -1, nullptr, nullptr, nullptr, nullptr, launches);
+        if (rc) return rc;
+    }
+    if (want(PC_SAMPLE) && !fold_argmax) {
+        ce = slab_argmax ? launch_argmax_finish(amax_val_, amax_idx_, nslabs, lm_rows, next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1, stream_, pdl_)
+                         : launch_argmax_finish(lg, nullptr, V_, lm_rows, next_dev, feed_dev, pos_dev, hist_dev, max_seq_ + 1, stream_, pdl_);
+        if (ce != cudaSuccess) return cuda_fail(ce, "argmax_finish");
+        ++*launches;
     }
     return HM_OK;
 }
@@ -1455,7 +1471,17 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
     // GGUF models run a chunk's projections as 8-row groups of the quantised kernels, launched back to back: the groups after
     // the first find the projection's weights in the L2, and attention, embedding and LM head run once per chunk
     const int chunk = (use_tc_ || quant_) ? TC_ROWS : MAX_M;
-    for (int c0 = 0; c0 < n; c0 += chunk) {
+    WidePlan plan;
+    if (const int wrc = plan_wide(st + n, st + 2 * n, n, &plan)) return wrc;
+    const int wide_rows = plan.rows;
+    for (const WidePass& w : plan.passes) {
+        const bool last = w.row0 + w.rows >= n;
+        int rc = enqueue_wide(w, pf_tokens_ + w.row0, pf_pos_ + w.row0, pf_seq_ + w.row0, &launches);
+        if (rc == HM_OK && last)
+            rc = enqueue_logits(wide_.h + (size_t)(w.rows - 1) * H_, 1, false, false, next_dev_ + seq, tokens_dev_ + seq, pos_dev_ + seq, hist_dev_ + (size_t)seq * (max_seq_ + 1), &launches);
+        if (rc) return rc;
+    }
+    for (int c0 = wide_rows; c0 < n; c0 += chunk) {
         const int mc = std::min(chunk, n - c0);
         const bool last = c0 + mc >= n;
         pass_longest_ = len0 + c0 + mc;

@@ -12,6 +12,7 @@
 
 #include "../../include/homura_b200.h"
 #include "common.cuh"
+#include "attn_prefill.h"
 #include "gla.h"
 #include "gqa_attn.h"
 #include "latent_attn.h"
@@ -124,6 +125,19 @@ struct ArgmaxFold {
     int hist_stride;
 };
 
+// A pass over many rows of prompts (engine_wide.cu): rows [row0, row0 + rows) of the call.
+struct WidePass {
+    struct Group { int tile0, tiles, block0, blocks; };  // launches of the prompt attention: parts of the call's tables
+    struct Range { int row0, rows; };                    // rows of short runs, within the pass: the decode attention
+    int row0 = 0, rows = 0;
+    std::vector<Group> groups;
+    std::vector<Range> singles;
+};
+struct WidePlan {
+    std::vector<WidePass> passes;
+    int rows = 0;  // rows that they cover; what is left at the end of the call is few
+};
+
 class Engine {
    public:
     // strict_f32: projections on the f32 streaming kernels only (no tensor-core copies of the weights)
@@ -177,6 +191,14 @@ class Engine {
     // Enqueue one pass over M rows (decode: one row per sequence; prefill: a chunk of one
     // sequence).  lm_row0/lm_rows select the rows that go through the LM head.
     int enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_pos, const int32_t* row_seq, int lm_row0, int lm_rows, bool advance, uint32_t* next_dev, uint32_t* feed_dev, int32_t* pos_dev, uint32_t* hist_dev, int* launches);
+    int enqueue_logits(const float* x, int lm_rows, bool whole_pass, bool packed, uint32_t* next_dev, uint32_t* feed_dev, int32_t* pos_dev, uint32_t* hist_dev, int* launches);
+    AttnArgs attn_args(int l, int M, const float* q, const int32_t* row_pos, const int32_t* row_seq) const;
+    // passes over many rows (engine_wide.cu)
+    bool wide_fits() const;
+    bool ensure_wide(int rows);
+    int plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan);
+    int enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches);
+    void free_wide();
     int enqueue_linear(const LinearW& L, int M, const float* x, int ldx, int pro, const float* norm_w, int epi, float* y, int ldy, const float* bias, const float* resid, int layer, const int32_t* row_pos, const int32_t* row_seq, float* amax_val, int32_t* amax_idx, int* launches, const struct ArgmaxFold* fold = nullptr, const LinOpt* opt = nullptr);
     // listed designs (engine_listed.cu)
     int load_listed_tensor(const std::string& name, int dtype, const int64_t* shape, int ndim, const void* host, size_t nbytes);
@@ -315,6 +337,18 @@ class Engine {
     bool att_cluster_ = true;
     int* err_flag_ = nullptr;
     unsigned int* fin_ticket_ = nullptr;  // ticket of the LM head's folded argmax
+
+    // passes over many rows: activations, activation images (gemm_wide.h), partial tiles, staged keys and values, tables
+    struct Wide {
+        int cap = 0;                     // rows
+        float *h = nullptr, *q = nullptr, *ss = nullptr, *ss2 = nullptr;
+        unsigned char *x = nullptr, *x2 = nullptr, *att = nullptr, *act = nullptr;
+        float* part = nullptr;
+        unsigned char* staged = nullptr;
+        size_t staged_bytes = 0;
+        int32_t *tables = nullptr, *tables_host = nullptr;
+        size_t table_words = 0, tiles_at = 0;
+    } wide_;
 
     // listed designs
     float *mix_raw_ = nullptr, *qlat_ = nullptr, *ctx_ = nullptr;  // input projection, queries in latent space, attention result in latent space

@@ -112,23 +112,38 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
     }
     uint32_t *p_tok = st_pin_, *p_pos = p_tok + st_rows_, *p_seq = p_pos + st_rows_, *p_want = p_seq + st_rows_, *p_next = p_want + st_rows_, *p_len = p_next + st_rows_;
     const int chunk = std::min(TC_ROWS, scratch_rows_);
-    std::vector<int> pass_wants((rows + chunk - 1) / chunk, 0), pass_longest(pass_wants.size(), 0);
     size_t r = 0, q = 0;
     for (int i = 0; i < n; ++i) {
         const hm_step_entry& e = entries[i];
-        int w = 0;
         for (int k = 0; k < e.n_tokens; ++k, ++r) {
             p_tok[r] = e.tokens[k];
             p_pos[r] = (uint32_t)(len_[e.seq] + k);
             p_seq[r] = (uint32_t)e.seq;
-            pass_longest[r / chunk] = std::max(pass_longest[r / chunk], len_[e.seq] + k + 1);
+        }
+        p_len[2 * i] = (uint32_t)(len_[e.seq] + e.n_tokens);
+    }
+    WidePlan plan;
+    if (const int wrc = plan_wide(p_pos, p_seq, (int)rows, &plan)) return wrc;
+    // passes: the wide ones, then chunks; wanted rows as indices within their pass
+    struct Pass { size_t row0; int rows, wants, longest; };
+    std::vector<Pass> passes;
+    for (const WidePass& w : plan.passes) passes.push_back({(size_t)w.row0, w.rows, 0, 0});
+    for (size_t c0 = plan.rows; c0 < rows; c0 += chunk) passes.push_back({c0, (int)std::min<size_t>(chunk, rows - c0), 0, 0});
+    r = 0;
+    size_t at = 0;
+    for (int i = 0; i < n; ++i) {
+        const hm_step_entry& e = entries[i];
+        int w = 0;
+        for (int k = 0; k < e.n_tokens; ++k, ++r) {
+            while (r >= passes[at].row0 + passes[at].rows) ++at;
+            Pass& p = passes[at];
+            p.longest = std::max(p.longest, len_[e.seq] + k + 1);
             if (w < e.n_want && e.want[w] == k) {
-                p_want[q++] = (uint32_t)(r % chunk);
-                pass_wants[r / chunk]++;
+                p_want[q++] = (uint32_t)(r - p.row0);
+                p.wants++;
                 ++w;
             }
         }
-        p_len[2 * i] = (uint32_t)(len_[e.seq] + e.n_tokens);
     }
     HM_CUDA(cudaMemcpyAsync(st_tokens_, p_tok, rows * 4, cudaMemcpyHostToDevice, stream_));
     HM_CUDA(cudaMemcpyAsync(st_pos_, p_pos, rows * 4, cudaMemcpyHostToDevice, stream_));
@@ -139,10 +154,27 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
     size_t done = 0;
     tap_ = hidden;
     tap_rows_ = rows;
-    for (size_t c0 = 0, pass = 0; c0 < rows && rc == HM_OK; c0 += chunk, ++pass) {
-        const int mc = (int)std::min<size_t>(chunk, rows - c0), nw = logits || greedy ? pass_wants[pass] : 0;
+    auto logits_out = [&](int nw) -> int {  // the wanted rows that the pass enqueued last left in logits_
+        if (!logits || !nw) return HM_OK;
+        const cudaError_t ce = cudaMemcpyAsync(land + done * V_, logits_, (size_t)nw * V_ * 4, cudaMemcpyDeviceToHost, stream_);
+        return ce == cudaSuccess ? HM_OK : cuda_fail(ce, "logits copy");
+    };
+    for (size_t i = 0; i < passes.size() && rc == HM_OK; ++i) {
+        const size_t c0 = passes[i].row0;
+        const int mc = passes[i].rows, nw = logits || greedy ? passes[i].wants : 0;
         tap_row0_ = c0;
-        pass_longest_ = pass_longest[pass];
+        if (i < plan.passes.size()) {
+            rc = enqueue_wide(plan.passes[i], st_tokens_ + c0, st_pos_ + c0, st_seq_ + c0, &launches);
+            for (int w = 0; w < nw && rc == HM_OK; w += chunk) {
+                const int g = std::min(chunk, nw - w);
+                const cudaError_t ce = launch_gather_rows(wide_.h, st_want_ + done, g, H_, hsel_, stream_, pdl_);
+                rc = ce == cudaSuccess ? enqueue_logits(hsel_, g, false, false, st_next_ + done, nullptr, nullptr, nullptr, &launches) : cuda_fail(ce, "gather_rows");
+                if (rc == HM_OK) rc = logits_out(g);
+                done += g;
+            }
+            continue;
+        }
+        pass_longest_ = passes[i].longest;
         pass_runs_.clear();
         for (int m = 0; m < mc; ++m) {  // a sequence's tokens are consecutive, so its rows within the pass are one run
             if (m > 0 && p_seq[c0 + m] == p_seq[c0 + m - 1]) pass_runs_.back().second++;
@@ -150,10 +182,7 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
         }
         lm_pick_ = nw ? st_want_ + done : nullptr;
         rc = enqueue_pass(mc, st_tokens_ + c0, st_pos_ + c0, st_seq_ + c0, 0, nw, false, st_next_ + done, nullptr, nullptr, nullptr, &launches);
-        if (rc == HM_OK && nw && logits) {
-            const cudaError_t ce = cudaMemcpyAsync(land + done * V_, logits_, (size_t)nw * V_ * 4, cudaMemcpyDeviceToHost, stream_);
-            if (ce != cudaSuccess) rc = cuda_fail(ce, "logits copy");
-        }
+        if (rc == HM_OK) rc = logits_out(nw);
         done += nw;
     }
     pass_runs_.clear();

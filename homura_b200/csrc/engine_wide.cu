@@ -1,0 +1,244 @@
+// Passes over many rows of prompts (65 to 2048) on the uniform bf16 stacks: every weight is read once per pass instead of once per 64
+// rows, projections run on the many-row GEMM (gemm_wide.cu) and runs of a sequence's rows on the prompt attention (attn_prefill.cu).
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <vector>
+
+#include "engine.h"
+#include "engine_util.h"
+#include "gemm_tc.h"
+#include "gemm_wide.h"
+
+namespace hm {
+
+// Runs shorter than this go to the decode attention, row by row: a tile of the prompt attention costs as much for one row as for 64,
+// and its context is staged first.
+constexpr int WIDE_MIN_RUN = 8;
+// Staged keys and values of one launch at most (one sequence may take more).
+constexpr size_t WIDE_STAGED = 512u << 20;
+
+bool Engine::wide_fits() const {
+    if (spec_.listed() || quant_ || !use_tc_ || H_ % 128 != 0 || I_ % 64 != 0 || page_tokens_ != 16) return false;
+    for (const LayerW& l : layers_)
+        if (!l.qkv.tc || !l.o.tc || !l.gu.tc || !l.down.tc) return false;
+    return true;
+}
+
+void Engine::free_wide() {
+    for (void* p : {(void*)wide_.h, (void*)wide_.q, (void*)wide_.ss, (void*)wide_.ss2, (void*)wide_.x, (void*)wide_.x2, (void*)wide_.att, (void*)wide_.act, (void*)wide_.part, (void*)wide_.staged, (void*)wide_.tables})
+        if (p) cudaFree(p);
+    if (wide_.tables_host) cudaFreeHost(wide_.tables_host);
+    wide_ = Wide();
+}
+
+// Scratch of a pass over `rows` rows (the stream is idle).  False without memory for it: the caller then takes passes of 64 rows.
+bool Engine::ensure_wide(int rows) {
+    if (rows <= wide_.cap) return true;
+    const int cap = std::min(WIDE_ROWS, (rows + 511) / 512 * 512), blocks = wide_blocks(cap);
+    size_t part = 1;
+    for (int b = 1; b <= blocks; ++b)
+        for (const LinearW* w : {&layers_[0].qkv, &layers_[0].o, &layers_[0].gu, &layers_[0].down})
+            part = std::max(part, wide_split(b * WIDE_BLOCK, w->K, w->N, w == &layers_[0].gu ? EPI_SWIGLU : EPI_STORE, sm_count_).part_floats);
+    free_wide();
+    auto get = [&](auto** p, size_t count) { return cudaMalloc((void**)p, count * sizeof(**p)) == cudaSuccess; };
+    const bool ok = get(&wide_.h, (size_t)cap * H_) && get(&wide_.q, (size_t)cap * qdim_) && get(&wide_.ss, (size_t)(H_ / 128) * cap) && get(&wide_.ss2, (size_t)(H_ / 128) * cap) &&
+                    get(&wide_.x, blocks * wide_block_bytes(H_)) && get(&wide_.x2, blocks * wide_block_bytes(H_)) && get(&wide_.att, blocks * wide_block_bytes(qdim_)) && get(&wide_.act, blocks * wide_block_bytes(I_)) &&
+                    get(&wide_.part, part);
+    if (!ok) {
+        cudaGetLastError();
+        free_wide();
+        return false;
+    }
+    wide_.cap = cap;
+    return true;
+}
+
+// Rows from which a call takes wide passes: more than one 64-row pass.  Prompts of 96 rows (two passes of the 64-row kernels): 0.5 B
+// 2.44 -> 1.83 ms, 1.5 B 4.28 -> 3.08; of 128: 2.63 -> 2.00, 4.64 -> 3.23.
+// Cuts the n rows of a call (host arrays: position and sequence of each; a sequence's rows are consecutive) into wide passes and sends
+// the tables of their attention to the device.  No passes where the rows are few or the model has no wide path.
+int Engine::plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan) {
+    plan->passes.clear();
+    plan->rows = 0;
+    if (n <= TC_ROWS || !wide_fits()) return HM_OK;
+    const int n_pass = (n + WIDE_ROWS - 1) / WIDE_ROWS;
+    const int per = std::min(WIDE_ROWS, ((n + n_pass - 1) / n_pass + WIDE_BLOCK - 1) / WIDE_BLOCK * WIDE_BLOCK);
+    if (!ensure_wide(std::min(per, n))) return HM_OK;
+    const size_t block_bytes = prefill_block_bytes(kvh_, hd_, kv_bf16_);
+    const int budget = (int)std::max<size_t>(1, WIDE_STAGED / block_bytes);
+    std::vector<PrefillTile> tiles;
+    std::vector<PrefillBlock> blocks;
+    int most = 0;
+    while (n - plan->rows > TC_ROWS) {
+        WidePass p;
+        p.row0 = plan->rows;
+        p.rows = std::min(per, n - p.row0);
+        auto close = [&]() {  // the longest tiles first, so that the last CTAs of the launch are short
+            WidePass::Group& g = p.groups.back();
+            g.tiles = (int)tiles.size() - g.tile0;
+            g.blocks = (int)blocks.size() - g.block0;
+            most = std::max(most, g.blocks);
+            std::stable_sort(tiles.begin() + g.tile0, tiles.end(), [](const PrefillTile& a, const PrefillTile& b) { return a.pos0 + a.rows > b.pos0 + b.rows; });
+        };
+        for (int r = 0; r < p.rows;) {
+            const uint32_t *ps = pos + p.row0 + r, *sq = seq + p.row0 + r;
+            int run = 1;
+            while (r + run < p.rows && sq[run] == sq[0]) ++run;
+            if (run < WIDE_MIN_RUN) {
+                if (!p.singles.empty() && p.singles.back().row0 + p.singles.back().rows == r) p.singles.back().rows += run;
+                else p.singles.push_back({r, run});
+            } else {
+                const int len = (int)ps[0] + run, nb = (len + PREFILL_TILE - 1) / PREFILL_TILE;
+                if (p.groups.empty() || (int)blocks.size() - p.groups.back().block0 + nb > budget) {
+                    if (!p.groups.empty()) close();
+                    p.groups.push_back({(int)tiles.size(), 0, (int)blocks.size(), 0});
+                }
+                const int b0 = (int)blocks.size() - p.groups.back().block0;
+                for (int b = 0; b < nb; ++b) blocks.push_back({(int32_t)sq[0], b * PREFILL_TILE, std::min(PREFILL_TILE, len - b * PREFILL_TILE), 0});
+                for (int t = 0; t < run; t += PREFILL_TILE) tiles.push_back({r + t, std::min(PREFILL_TILE, run - t), (int32_t)ps[0] + t, b0});
+            }
+            r += run;
+        }
+        if (!p.groups.empty()) close();
+        plan->rows += p.rows;
+        plan->passes.push_back(std::move(p));
+    }
+    static_assert(sizeof(PrefillTile) == 16 && sizeof(PrefillBlock) == 16, "table entries are four words");
+    const size_t words = 4 * (tiles.size() + blocks.size());
+    auto give_up = [&]() {  // without memory: passes of 64 rows
+        cudaGetLastError();
+        plan->passes.clear();
+        plan->rows = 0;
+        return HM_OK;
+    };
+    if (words > wide_.table_words) {
+        if (wide_.tables) cudaFree(wide_.tables);
+        if (wide_.tables_host) cudaFreeHost(wide_.tables_host);
+        wide_.tables = wide_.tables_host = nullptr;
+        wide_.table_words = 0;
+        const size_t cap = std::max<size_t>(4096, words + words / 2);
+        if (cudaMalloc((void**)&wide_.tables, cap * 4) != cudaSuccess || cudaMallocHost((void**)&wide_.tables_host, cap * 4) != cudaSuccess) return give_up();
+        wide_.table_words = cap;
+    }
+    if (most * block_bytes > wide_.staged_bytes) {
+        if (wide_.staged) cudaFree(wide_.staged);
+        wide_.staged = nullptr;
+        wide_.staged_bytes = 0;
+        const size_t bytes = std::max<size_t>(most * block_bytes, std::min<size_t>(WIDE_STAGED, 2 * most * block_bytes));
+        if (cudaMalloc((void**)&wide_.staged, bytes) != cudaSuccess) return give_up();
+        wide_.staged_bytes = bytes;
+    }
+    if (words) {
+        std::memcpy(wide_.tables_host, tiles.data(), tiles.size() * sizeof(PrefillTile));
+        wide_.tiles_at = 4 * tiles.size();
+        std::memcpy(wide_.tables_host + wide_.tiles_at, blocks.data(), blocks.size() * sizeof(PrefillBlock));
+        HM_CUDA(cudaMemcpyAsync(wide_.tables, wide_.tables_host, words * 4, cudaMemcpyHostToDevice, stream_));
+    }
+    return HM_OK;
+}
+
+// All layers of one pass; the residual stream is left in wide_.h.
+int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches) {
+    const int M = p.rows;
+    const float eps = (float)cfg_.rms_norm_eps;
+    cudaError_t ce = launch_embed_gather(embed_, embed_dtype_ == HM_BF16 ? 1 : 0, tokens, M, H_, V_, wide_.h, err_flag_, stream_, pdl_);
+    if (ce != cudaSuccess) return cuda_fail(ce, "embed_gather");
+    ce = launch_wide_pack(wide_.h, H_, M, H_, layers_[0].in_ln, eps, wide_.x, stream_, pdl_);
+    if (ce != cudaSuccess) return cuda_fail(ce, "activation pack");
+    *launches += 2;
+    for (int l = 0; l < L_; ++l) {
+        const LayerW& w = layers_[l];
+        const KvDesc kv{k_pool_[l], v_pool_[l], page_table_, max_pages_, page_tokens_, kvh_, hd_, kv_bf16_ ? 1 : 0};
+        auto project = [&](const LinearW& L, const unsigned char* xp, int epi, WideArgs a) {
+            a.W = L.tc;
+            a.K = L.K;
+            a.N = L.N;
+            a.M = M;
+            a.xp = xp;
+            a.epi = epi;
+            a.eps = eps;
+            a.ss_parts = H_ / 128;
+            a.ss_ld = wide_.cap;
+            a.part = wide_.part;
+            a.err_flag = err_flag_;
+            return launch_gemm_wide(a, sm_count_, stream_, pdl_, launches);
+        };
+        WideArgs qkv{};
+        qkv.bias = w.qkv_bias;
+        qkv.y = wide_.q;
+        qkv.ldy = qdim_;
+        qkv.ss_in = l > 0 ? wide_.ss : nullptr;  // the first layer's rows were normalised when they were packed
+        qkv.q_dim = qdim_;
+        qkv.kv_dim = kvdim_;
+        qkv.hd = hd_;
+        qkv.has_qk_norm = cfg_.has_qk_norm;
+        qkv.q_norm_w = w.q_norm;
+        qkv.k_norm_w = w.k_norm;
+        qkv.rope_cos = rope_cos_;
+        qkv.rope_sin = rope_sin_;
+        qkv.row_pos = row_pos;
+        qkv.row_seq = row_seq;
+        qkv.kv = kv;
+        ce = project(w.qkv, wide_.x, EPI_QKV_ROPE, qkv);
+        if (ce != cudaSuccess) return cuda_fail(ce, "wide QKV projection");
+        for (const WidePass::Group& g : p.groups) {
+            PrefillArgs a{};
+            a.kv = kv;
+            a.heads = heads_;
+            a.scale = (float)(1.0 / std::sqrt((double)hd_));
+            a.q = wide_.q;
+            a.staged = wide_.staged;
+            a.tiles = reinterpret_cast<const PrefillTile*>(wide_.tables) + g.tile0;
+            a.blocks = reinterpret_cast<const PrefillBlock*>(wide_.tables + wide_.tiles_at) + g.block0;
+            a.n_tiles = g.tiles;
+            a.n_blocks = g.blocks;
+            a.xp_out = wide_.att;
+            a.xp_block = wide_block_bytes(qdim_);
+            a.err_flag = err_flag_;
+            ce = launch_attn_prefill(a, stream_, pdl_, launches);
+            if (ce != cudaSuccess) return cuda_fail(ce, "prompt attention");
+        }
+        for (const WidePass::Range& r : p.singles)
+            for (int r0 = r.row0; r0 < r.row0 + r.rows; r0 += scratch_rows_) {
+                const int n = std::min(scratch_rows_, r.row0 + r.rows - r0);
+                AttnArgs at = attn_args(l, n, wide_.q + (size_t)r0 * qdim_, row_pos + r0, row_seq + r0);
+                at.xp_out = wide_.att;
+                at.xp_mpad = WIDE_BLOCK;
+                at.xp_block = wide_block_bytes(qdim_);
+                at.xp_row0 = r0;
+                ce = launch_attn_decode(at, n, kv_bf16_, stream_, pdl_);
+                if (ce != cudaSuccess) return cuda_fail(ce, "attention launch");
+                ++*launches;
+            }
+        WideArgs o{};
+        o.resid = wide_.h;
+        o.y = wide_.h;
+        o.ldy = H_;
+        o.xp_out = wide_.x2;
+        o.next_norm_w = w.post_ln;
+        o.ss_out = wide_.ss2;
+        ce = project(w.o, wide_.att, EPI_STORE, o);
+        if (ce != cudaSuccess) return cuda_fail(ce, "wide output projection");
+        WideArgs gu{};
+        gu.ss_in = wide_.ss2;
+        gu.xp_out = wide_.act;
+        ce = project(w.gu, wide_.x2, EPI_SWIGLU, gu);
+        if (ce != cudaSuccess) return cuda_fail(ce, "wide gate/up projection");
+        WideArgs dn{};
+        dn.resid = wide_.h;
+        dn.y = wide_.h;
+        dn.ldy = H_;
+        if (l + 1 < L_) {
+            dn.xp_out = wide_.x;
+            dn.next_norm_w = layers_[l + 1].in_ln;
+            dn.ss_out = wide_.ss;
+        }
+        ce = project(w.down, wide_.act, EPI_STORE, dn);
+        if (ce != cudaSuccess) return cuda_fail(ce, "wide down projection");
+        if (tap_) HM_CUDA(cudaMemcpyAsync(tap_ + ((size_t)l * tap_rows_ + tap_row0_) * H_, wide_.h, (size_t)M * H_ * 4, cudaMemcpyDeviceToHost, stream_));
+    }
+    return HM_OK;
+}
+
+}  // namespace hm
