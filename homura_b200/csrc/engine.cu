@@ -3,6 +3,7 @@
 #include "sandwich.h"
 #include "engine_util.h"
 #include "gemm_tc.h"
+#include "gemm_wide.h"
 #include "kquant.h"
 #include "sampler.h"
 
@@ -118,7 +119,7 @@ Engine::~Engine() {
         for (float* p : {l.in_ln, l.post_ln, l.qkv_bias, l.q_norm, l.k_norm, l.shift, l.ls1, l.ls2, l.latent_norm, l.v_mix, l.rel, l.correction, l.in_bias, l.sink, l.conv_w, l.lin_norm, l.lin_up, l.lin_bias, l.norm1b, l.norm2b, l.left_out, l.right_out, l.talk, l.temp, l.gu_bias, l.down_bias, l.lin_conv_w, l.lin_rate, l.lin_up_g, l.lin_decay}) fr(p);
     for (auto& l : layers_) { fr(l.router); fr(l.exp_gu); fr(l.exp_down); fr(l.turns); }
     fr(turns_); fr(bigram_);
-    each_linear([&](LinearW& w) { fr(w.slabs); fr(w.tc); fr(w.scales); fr(w.codes); fr(w.kq_data); fr(w.kq_tile_type); });
+    each_linear([&](LinearW& w) { fr(w.slabs); fr(w.tc); fr(w.wide); fr(w.scales); fr(w.codes); fr(w.kq_data); fr(w.kq_tile_type); });
     free_listed();
     free_wide();
     free_listed_cache();
@@ -232,6 +233,20 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
         }
         if (ce == cudaSuccess) ce = launch_split_blocks((const uint8_t*)tmp, n_part, K, q4, n_off, interleave_which, L.scales, L.codes, stream_, rope_hd);
         quant_ = true;
+        // a second copy for prompts (4 or 6 bytes per weight); without the memory for it prompts run in passes of 64 rows
+        if (ce == cudaSuccess && use_tc_ && &L != &lm_head_ && K % 64 == 0) {
+            if (!L.wide && L.loaded_parts == 0) {
+                L.wide_terms = wide_quant_terms(q4);
+                const size_t bytes = tc_packed_elems(K, N_total) * 2 * L.wide_terms;
+                if (cudaMalloc(&L.wide, bytes) == cudaSuccess) {
+                    ce = cudaMemsetAsync(L.wide, 0, bytes, stream_);
+                } else {
+                    cudaGetLastError();
+                    L.wide = nullptr;
+                }
+            }
+            if (ce == cudaSuccess && L.wide) ce = launch_wide_pack_quant((const uint8_t*)tmp, n_part, K, q4, L.wide, n_off, interleave_which, stream_);
+        }
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream_);
     cudaFree(tmp);

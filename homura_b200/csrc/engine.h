@@ -31,6 +31,8 @@ struct LinearW {
     int kind = -1;           // HM_BF16 (slab layout) | HM_Q8_0 | HM_Q4_0 (split scales + codes)
     uint16_t* slabs = nullptr;
     uint16_t* tc = nullptr;  // second copy in the tensor-core tile layout (gemm_tc.h), used for passes over more than 8 rows
+    uint16_t* wide = nullptr;  // Q8_0 / Q4_0: the weights as bf16 terms (gemm_wide.h), for prompts of more than 64 rows
+    int wide_terms = 0;
     uint16_t* scales = nullptr;
     uint8_t* codes = nullptr;
     uint8_t* kq_data = nullptr;       // K-quants (kind HM_Q4_K stands for the family): tiled super-blocks, kquant.h

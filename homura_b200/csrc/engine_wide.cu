@@ -1,4 +1,4 @@
-// Passes over many rows of prompts (65 to 2048) on the uniform bf16 stacks: every weight is read once per pass instead of once per 64
+// Passes over many rows of prompts (65 to 2048) on the uniform stacks (bf16, Q8_0 and Q4_0 weights): every weight is read once per pass instead of once per 64
 // rows, projections run on the many-row GEMM (gemm_wide.cu) and runs of a sequence's rows on the prompt attention (attn_prefill.cu).
 #include <algorithm>
 #include <cmath>
@@ -19,9 +19,10 @@ constexpr int WIDE_MIN_RUN = 8;
 constexpr size_t WIDE_STAGED = 512u << 20;
 
 bool Engine::wide_fits() const {
-    if (spec_.listed() || quant_ || !use_tc_ || H_ % 128 != 0 || I_ % 64 != 0 || page_tokens_ != 16) return false;
+    if (spec_.listed() || !use_tc_ || H_ % 128 != 0 || I_ % 64 != 0 || page_tokens_ != 16) return false;
     for (const LayerW& l : layers_)
-        if (!l.qkv.tc || !l.o.tc || !l.gu.tc || !l.down.tc) return false;
+        for (const LinearW* w : {&l.qkv, &l.o, &l.gu, &l.down})
+            if (!w->tc && !w->wide) return false;
     return true;
 }
 
@@ -39,7 +40,7 @@ bool Engine::ensure_wide(int rows) {
     size_t part = 1;
     for (int b = 1; b <= blocks; ++b)
         for (const LinearW* w : {&layers_[0].qkv, &layers_[0].o, &layers_[0].gu, &layers_[0].down})
-            part = std::max(part, wide_split(b * WIDE_BLOCK, w->K, w->N, w == &layers_[0].gu ? EPI_SWIGLU : EPI_STORE, sm_count_).part_floats);
+            part = std::max(part, wide_split(b * WIDE_BLOCK, w->K, w->N, w->tc ? 1 : w->wide_terms, w == &layers_[0].gu ? EPI_SWIGLU : EPI_STORE, sm_count_).part_floats);
     free_wide();
     auto get = [&](auto** p, size_t count) { return cudaMalloc((void**)p, count * sizeof(**p)) == cudaSuccess; };
     const bool ok = get(&wide_.h, (size_t)cap * H_) && get(&wide_.q, (size_t)cap * qdim_) && get(&wide_.ss, (size_t)(H_ / 128) * cap) && get(&wide_.ss2, (size_t)(H_ / 128) * cap) &&
@@ -55,7 +56,7 @@ bool Engine::ensure_wide(int rows) {
 }
 
 // Rows from which a call takes wide passes: more than one 64-row pass.  Prompts of 96 rows (two passes of the 64-row kernels): 0.5 B
-// 2.44 -> 1.83 ms, 1.5 B 4.28 -> 3.08; of 128: 2.63 -> 2.00, 4.64 -> 3.23.
+// 2.44 -> 1.83 ms, 1.5 B 4.28 -> 3.08; of 128: 2.63 -> 2.00, 4.64 -> 3.23; of 65 on TinyLlama Q8_0 4.23 -> 2.87, Q4_0 4.64 -> 2.52.
 // Cuts the n rows of a call (host arrays: position and sequence of each; a sequence's rows are consecutive) into wide passes and sends
 // the tables of their attention to the device.  No passes where the rows are few or the model has no wide path.
 int Engine::plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan) {
@@ -151,7 +152,8 @@ int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_
         const LayerW& w = layers_[l];
         const KvDesc kv{k_pool_[l], v_pool_[l], page_table_, max_pages_, page_tokens_, kvh_, hd_, kv_bf16_ ? 1 : 0};
         auto project = [&](const LinearW& L, const unsigned char* xp, int epi, WideArgs a) {
-            a.W = L.tc;
+            a.W = L.tc ? L.tc : L.wide;
+            a.w_terms = L.tc ? 1 : L.wide_terms;
             a.K = L.K;
             a.N = L.N;
             a.M = M;

@@ -12,12 +12,15 @@
 //     per addition).  Accumulators therefore cover CHUNK k-blocks only; two of them (256 TMEM columns each) alternate,
 //     and eight warps add the finished one to f32 registers (round to nearest) while the other is being filled.  A thread owns
 //     one row and 128 consecutive features, so that norms, rotation and gating need no exchange between threads.
+//   * Q8_0 and Q4_0 weights (f16 scale times code: 19 and 15 bits) come as three and two bf16 terms, exactly, and take the six and five
+//     products that reach 2^-24; a weight tile then serves the activation terms that it meets, the small products first.
 //   * the gated activations of a whole contraction leave from the same registers.  Everything else goes as f32 partial tiles to scratch
 //     (the L2) and a second launch (wide_finish_kernel) adds the parts of a split contraction in their order and does the epilogue, a
 //     warp per row of 128 features: the outputs of a unit that no other unit of its CTA follows would otherwise leave at the pace of
 //     eight warps (15 us for 128 x 256 residuals, images and sums of squares; 3 us for the partial tile).
 // Measured: gate/up of 2048 rows (K 1536, N 17920) 287 us = 1.18 PFLOP/s of bf16 products, down (K 8960, N 1536) 119 + 14 us, where the
-// 64-row launches took 32 x 15.0 and 32 x 13.2 us; a prompt of 1999 tokens on the 0.5 B stack 52.1 -> 9.2 ms.  What bounds it is the
+// 64-row launches took 32 x 15.0 and 32 x 13.2 us; a prompt of 1999 tokens on the 0.5 B stack 52.1 -> 9.2 ms,
+// 1021 tokens on TinyLlama Q8_0 60.1 -> 12.1 ms and Q4_0 66.8 -> 10.7 ms (64-row launches on digit planes and integer MMAs before).  What bounds it is the
 // traffic between L2 and shared memory (80 KB per k-block and SM) and the read-back of the accumulators: one per two k-blocks costs 12 %
 // against one per four, which leaves 1.8 times the error.
 #include <algorithm>
@@ -35,7 +38,9 @@ constexpr int WB_TILE = 128 * BK * 2;        // one block of 128 features
 constexpr int W_SLOT = 2 * WB_TILE;          // 256 features x 64 k
 constexpr int X_SLOT = WIDE_BLOCK * BK * 2;  // one term of 128 rows x 64 k
 constexpr int W_SLOTS = 3, X_SLOTS = 6;
-constexpr int CHUNK = 2;                     // k-blocks per accumulator
+// k-blocks per accumulator
+template <int WT>
+constexpr int CHUNK = WT == 1 ? 2 : 1;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 64 + EPI_WARPS * 32;
 constexpr int STAGE = 32 * 32 * 4;           // an epilogue warp's 32 rows x 32 columns on their way to or from global memory
@@ -135,8 +140,8 @@ __device__ __forceinline__ void epi_swiglu(const WideArgs& a, float (&acc)[128],
     }
 }
 
-// GLU: gated activations of unsplit contractions; else partial tiles.
-template <bool GLU>
+// GLU: gated activations of unsplit contractions; else partial tiles.  WT: terms of a weight; term w meets the activation terms 2 - w .. 0.
+template <bool GLU, int WT>
 __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a) {
     extern __shared__ __align__(1024) unsigned char dsm[];
     __shared__ WideShared sh;
@@ -164,43 +169,38 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
     if (warp == 0) {
         if (lane == 0) {
             const unsigned char* W = reinterpret_cast<const unsigned char*>(a.W);
-            const size_t nb_bytes = (size_t)a.kblocks * WB_TILE, rb_bytes = (size_t)a.kblocks * 3 * X_SLOT;
+            const size_t nb_bytes = (size_t)a.kblocks * WT * WB_TILE, rb_bytes = (size_t)a.kblocks * 3 * X_SLOT;
             uint32_t wi = 0, xi = 0;  // slots used so far
-            bool ok = true;
-            // weights do not depend on the launch in front: the first slots are filled before its end
-            uint32_t ahead = 0;
-            {
-                const Unit t = unit_at(a, blockIdx.x);
+            auto load_w = [&](const Unit& t, int i, uint32_t s) {  // the unit's i-th weight tile, the small terms of a k-block first
                 const bool two = 2 * t.tile + 1 < a.nblocks;
-                const unsigned char* w0 = W + (size_t)(2 * t.tile) * nb_bytes;
-                for (; ahead < (uint32_t)min(W_SLOTS, t.kb1 - t.kb0); ++ahead) {
-                    unsigned char* dst = wring + (size_t)ahead * W_SLOT;
-                    mb_expect_tx(&sh.wfull[ahead], two ? W_SLOT : WB_TILE);
-                    bulk_copy(dst, w0 + (size_t)(t.kb0 + ahead) * WB_TILE, WB_TILE, &sh.wfull[ahead]);
-                    if (two) bulk_copy(dst + WB_TILE, w0 + nb_bytes + (size_t)(t.kb0 + ahead) * WB_TILE, WB_TILE, &sh.wfull[ahead]);
-                }
-            }
+                const unsigned char* src = W + (size_t)(2 * t.tile) * nb_bytes + ((size_t)(t.kb0 + i / WT) * WT + (WT - 1 - i % WT)) * WB_TILE;
+                unsigned char* dst = wring + (size_t)s * W_SLOT;
+                mb_expect_tx(&sh.wfull[s], two ? W_SLOT : WB_TILE);
+                bulk_copy(dst, src, WB_TILE, &sh.wfull[s]);
+                if (two) bulk_copy(dst + WB_TILE, src + nb_bytes, WB_TILE, &sh.wfull[s]);
+            };
+            // weights do not depend on the launch in front: the first slots are filled before its end
+            const Unit first = unit_at(a, blockIdx.x);
+            const uint32_t ahead = min(W_SLOTS, (first.kb1 - first.kb0) * WT);
+            for (uint32_t i = 0; i < ahead; ++i) load_w(first, (int)i, i);
             pdl_wait();
+            bool ok = true;
             for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit t = unit_at(a, u);
-                const bool two = 2 * t.tile + 1 < a.nblocks;
-                const unsigned char *w0 = W + (size_t)(2 * t.tile) * nb_bytes, *x0 = a.xp + (size_t)t.rb * rb_bytes;
-                for (int kb = t.kb0; kb < t.kb1 && ok; ++kb) {
+                const unsigned char* x0 = a.xp + (size_t)t.rb * rb_bytes;
+                for (int i = 0; i < (t.kb1 - t.kb0) * WT && ok; ++i, ++wi) {
                     const uint32_t s = wi % W_SLOTS;
                     if (wi >= W_SLOTS) ok = mb_wait(&sh.wempty[s], ((wi / W_SLOTS) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
                     if (!ok) break;
-                    if (wi >= ahead) {
-                        mb_expect_tx(&sh.wfull[s], two ? W_SLOT : WB_TILE);
-                        bulk_copy(wring + (size_t)s * W_SLOT, w0 + (size_t)kb * WB_TILE, WB_TILE, &sh.wfull[s]);
-                        if (two) bulk_copy(wring + (size_t)s * W_SLOT + WB_TILE, w0 + nb_bytes + (size_t)kb * WB_TILE, WB_TILE, &sh.wfull[s]);
-                    }
-                    ++wi;
-                    for (int term = 2; term >= 0; --term, ++xi) {
+                    if (wi >= ahead) load_w(t, i, s);
+                    // the activation terms that this weight term is the first to meet
+                    const int w = WT - 1 - i % WT;
+                    for (int term = 2 - w; term >= (w == WT - 1 ? 0 : 2 - w); --term, ++xi) {
                         const uint32_t x = xi % X_SLOTS;
                         if (xi >= X_SLOTS) ok = mb_wait(&sh.xempty[x], ((xi / X_SLOTS) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
                         if (!ok) break;
                         mb_expect_tx(&sh.xfull[x], X_SLOT);
-                        bulk_copy(xring + (size_t)x * X_SLOT, x0 + ((size_t)kb * 3 + term) * X_SLOT, X_SLOT, &sh.xfull[x]);
+                        bulk_copy(xring + (size_t)x * X_SLOT, x0 + ((size_t)(t.kb0 + i / WT) * 3 + term) * X_SLOT, X_SLOT, &sh.xfull[x]);
                     }
                 }
             }
@@ -212,31 +212,36 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
             bool ok = true;
             for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit t = unit_at(a, u);
-                for (int kc = t.kb0; kc < t.kb1 && ok; kc += CHUNK, ++ci) {
+                for (int kc = t.kb0; kc < t.kb1 && ok; kc += CHUNK<WT>, ++ci) {
                     const uint32_t buf = ci & 1u, d = tmem + buf * 256u;
                     if (ci >= 2) ok = mb_wait(&sh.aempty[buf], ((ci >> 1) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     uint32_t more = 0;
-                    const int ke = min(t.kb1, kc + CHUNK);
-                    for (int kb = kc; kb < ke && ok; ++kb, ++wi) {
-                        const uint32_t s = wi % W_SLOTS;
-                        ok = mb_wait(&sh.wfull[s], (wi / W_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
-                        const uint32_t wa = s32(wring + (size_t)s * W_SLOT);
-                        for (int term = 0; term < 3 && ok; ++term, ++xi) {  // small terms first
-                            const uint32_t x = xi % X_SLOTS;
-                            ok = mb_wait(&sh.xfull[x], (xi / X_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
-                            if (!ok) break;
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t xa = s32(xring + (size_t)x * X_SLOT);
+                    const int ke = min(t.kb1, kc + CHUNK<WT>);
+                    for (int kb = kc; kb < ke && ok; ++kb, xi += 3) {
 #pragma unroll
-                            for (int ks = 0; ks < BK / 16; ++ks) {
-                                mma_f16(d, desc_sw128(xa + ks * 32), desc_sw128(wa + ks * 32), idesc, more);
-                                more = 1;
+                        for (int w = WT - 1; w >= 0; --w, ++wi) {
+                            const uint32_t s = wi % W_SLOTS;
+                            ok = ok && mb_wait(&sh.wfull[s], (wi / W_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
+                            const uint32_t wa = s32(wring + (size_t)s * W_SLOT);
+#pragma unroll
+                            for (int term = 2 - w; term >= 0; --term) {  // small products first
+                                // place of the term among the three of this k-block: in the order of their first use
+                                const uint32_t xn = xi + (WT == 1 ? 2 - term : WT == 2 ? (term == 2 ? 2 : 1 - term) : term), x = xn % X_SLOTS;
+                                if (w == WT - 1 || term == 2 - w) ok = ok && mb_wait(&sh.xfull[x], (xn / X_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
+                                if (!ok) break;
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                const uint32_t xa = s32(xring + (size_t)x * X_SLOT);
+#pragma unroll
+                                for (int ks = 0; ks < BK / 16; ++ks) {
+                                    mma_f16(d, desc_sw128(xa + ks * 32), desc_sw128(wa + ks * 32), idesc, more);
+                                    more = 1;
+                                }
+                                if (w == 0) mma_commit(&sh.xempty[x]);
                             }
-                            mma_commit(&sh.xempty[x]);
+                            if (ok) mma_commit(&sh.wempty[s]);
                         }
-                        if (ok) mma_commit(&sh.wempty[s]);
                     }
                     if (ok) mma_commit(&sh.afull[buf]);
                 }
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
 #pragma unroll
             for (int j = 0; j < 128; ++j) acc[j] = 0.f;
             bool ok = true;
-            for (int kc = t.kb0; kc < t.kb1; kc += CHUNK, ++ci) {
+            for (int kc = t.kb0; kc < t.kb1; kc += CHUNK<WT>, ++ci) {
                 const uint32_t buf = ci & 1u;
                 ok = __all_sync(0xffffffffu, mb_wait(&sh.afull[buf], (ci >> 1) & 1u, a.err_flag, &sh.abort_flag));
                 if (!ok) continue;
@@ -449,6 +454,34 @@ __global__ void __launch_bounds__(256) wide_pack_kernel(const float* __restrict_
     }
 }
 
+// a thread per eight consecutive inputs of a row
+__global__ void __launch_bounds__(256) wide_pack_quant_kernel(const uint8_t* __restrict__ blocks, int n_rows, int K, int q4, unsigned char* __restrict__ dst, int n_off, int interleave_which, int terms) {
+    const size_t total = (size_t)n_rows * (K / 8);
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const int n = (int)(i / (K / 8)), k = (int)(i % (K / 8)) * 8, c = (k & 31) >> 3;
+        const uint8_t* b = blocks + ((size_t)n * (K / 32) + k / 32) * (q4 ? 18 : 34);
+        const float d = f16_bits_to_f32((uint16_t)(b[0] | b[1] << 8));
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            if (q4) {  // byte j: element j in the low, element j + 16 in the high nibble
+                const uint8_t q = b[2 + (c & 1) * 8 + e];
+                v[e] = d * (float)((int)(c >= 2 ? q >> 4 : q & 15) - 8);
+            } else {
+                v[e] = d * (float)(int8_t)b[2 + c * 8 + e];
+            }
+        }
+        uint32_t w[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) bf16x2_split3(v[2 * e], v[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+        const int row = interleave_which >= 0 ? (n / 64) * 128 + interleave_which * 64 + n % 64 : n + n_off;
+        unsigned char* tile = dst + (((size_t)(row / 128) * (K / BK) + k / BK) * terms) * WB_TILE + (row % 128) * 128 + ((((k % BK) >> 3) ^ (row & 7)) << 4);
+#pragma unroll
+        for (int t = 0; t < 3; ++t)
+            if (t < terms) *reinterpret_cast<uint4*>(tile + (size_t)t * WB_TILE) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
+    }
+}
+
 template <typename F>
 cudaError_t launch(F* kernel, const WideArgs& a, dim3 grid, int threads, size_t smem, cudaStream_t st, bool pdl) {
     cudaLaunchConfig_t cfg = {};
@@ -464,6 +497,12 @@ cudaError_t launch(F* kernel, const WideArgs& a, dim3 grid, int threads, size_t 
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
+template <bool GLU, int WT>
+cudaError_t launch_product(const WideArgs& a, int sm_count, cudaStream_t st, bool pdl) {
+    const cudaError_t e = ensure_dyn_smem(gemm_wide_kernel<GLU, WT>, SMEM);
+    return e == cudaSuccess ? launch(gemm_wide_kernel<GLU, WT>, a, dim3((unsigned)std::min(a.units, sm_count)), THREADS, SMEM, st, pdl) : e;
+}
+
 template <int S>
 cudaError_t launch_finish(const WideArgs& a, cudaStream_t st, bool pdl) {
     const dim3 grid((unsigned)a.nblocks, (unsigned)((a.M + 31) / 32));
@@ -474,9 +513,10 @@ cudaError_t launch_finish(const WideArgs& a, cudaStream_t st, bool pdl) {
 
 }  // namespace
 
-WideSplit wide_split(int M, int K, int N, int epi, int sm_count) {
+WideSplit wide_split(int M, int K, int N, int w_terms, int epi, int sm_count) {
+    const double per_kb = w_terms == 1 ? 0.82 : w_terms == 2 ? 1.37 : 1.64;  // three, five and six products
     const int kb = (K + BK - 1) / BK, tiles = ((N + 127) / 128 + 1) / 2 * wide_blocks(M);
-    // Microseconds: rounds of units (0.82 per k-block, of a CTA's last unit also 3 for its partial tile), and the second launch, which
+    // Microseconds: rounds of units (0.82 per k-block of three products, of a CTA's last unit also 3 for its partial tile), and the second launch, which
     // reads the parts and writes ten bytes per output (6 TB/s in the L2, 4 us at least).
     int best = 1;
     double best_cost = 0;
@@ -484,7 +524,7 @@ WideSplit wide_split(int M, int K, int N, int epi, int sm_count) {
         const int per = (kb + s - 1) / s;
         const double rounds = (double)(((long)tiles * s + sm_count - 1) / sm_count);
         const bool parts = epi != EPI_SWIGLU || s > 1;
-        const double cost = rounds * (per * 0.82 + 0.5) + (parts ? 3.0 + std::max(4.0, (double)tiles * 128 * 256 * (4.0 * s + 10) / 6e6) : 6.0);
+        const double cost = rounds * (per * per_kb + 0.5) + (parts ? 3.0 + std::max(4.0, (double)tiles * 128 * 256 * (4.0 * s + 10) / 6e6) : 6.0);
         if (s == 1 || cost < best_cost) {
             best_cost = cost;
             best = s;
@@ -504,19 +544,27 @@ cudaError_t launch_gemm_wide(const WideArgs& a_in, int sm_count, cudaStream_t st
     a.nblocks = (a.N + 127) / 128;
     a.tiles = (a.nblocks + 1) / 2;
     a.row_blocks = wide_blocks(a.M);
-    a.kb_per = (a.kblocks + wide_split(a.M, a.K, a.N, a.epi, sm_count).split - 1) / wide_split(a.M, a.K, a.N, a.epi, sm_count).split;
+    const int split = wide_split(a.M, a.K, a.N, a.w_terms, a.epi, sm_count).split;
+    a.kb_per = (a.kblocks + split - 1) / split;
     a.split = (a.kblocks + a.kb_per - 1) / a.kb_per;
     a.units = a.tiles * a.row_blocks * a.split;
     const bool whole = a.epi == EPI_SWIGLU && a.split == 1;
     if (!whole && !a.part) return cudaErrorInvalidValue;
-    cudaError_t e = whole ? ensure_dyn_smem(gemm_wide_kernel<true>, SMEM) : ensure_dyn_smem(gemm_wide_kernel<false>, SMEM);
-    if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)std::min(a.units, sm_count));
     ++*launches;
-    e = whole ? launch(gemm_wide_kernel<true>, a, grid, THREADS, SMEM, st, pdl) : launch(gemm_wide_kernel<false>, a, grid, THREADS, SMEM, st, pdl);
+    const cudaError_t e = a.w_terms == 1   ? (whole ? launch_product<true, 1>(a, sm_count, st, pdl) : launch_product<false, 1>(a, sm_count, st, pdl))
+                          : a.w_terms == 2 ? (whole ? launch_product<true, 2>(a, sm_count, st, pdl) : launch_product<false, 2>(a, sm_count, st, pdl))
+                          : a.w_terms == 3 ? (whole ? launch_product<true, 3>(a, sm_count, st, pdl) : launch_product<false, 3>(a, sm_count, st, pdl))
+                                           : cudaErrorInvalidValue;
     if (e != cudaSuccess || whole) return e;
     ++*launches;
     return a.split == 1 ? launch_finish<1>(a, st, pdl) : a.split <= 4 ? launch_finish<4>(a, st, pdl) : launch_finish<8>(a, st, pdl);
+}
+
+cudaError_t launch_wide_pack_quant(const uint8_t* blocks, int n_rows, int K, bool q4, uint16_t* dst, int n_off, int interleave_which, cudaStream_t st) {
+    if (K % BK != 0 || n_rows < 1) return cudaErrorInvalidValue;
+    const size_t g = std::min<size_t>(((size_t)n_rows * (K / 8) + 255) / 256, 148 * 32);
+    wide_pack_quant_kernel<<<(unsigned)g, 256, 0, st>>>(blocks, n_rows, K, q4 ? 1 : 0, reinterpret_cast<unsigned char*>(dst), n_off, interleave_which, wide_quant_terms(q4));
+    return cudaGetLastError();
 }
 
 cudaError_t launch_wide_pack(const float* x, int ldx, int M, int K, const float* norm_w, float eps, unsigned char* xp, cudaStream_t st, bool pdl) {

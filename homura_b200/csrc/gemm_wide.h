@@ -16,7 +16,8 @@ __host__ __device__ inline size_t wide_block_bytes(int K) { return (size_t)((K +
 inline int wide_blocks(int M) { return (M + WIDE_BLOCK - 1) / WIDE_BLOCK; }
 
 struct WideArgs {
-    const uint16_t* W;        // weights as the tensor-core tiles of launch_pack_tc
+    const uint16_t* W;        // weights as the tensor-core tiles of launch_pack_tc, or of launch_wide_pack_quant:
+    int w_terms;              // bf16 terms per weight: 1; 2 or 3, the terms of a tile in a row
     int K, N, M;
     const unsigned char* xp;  // activation image
     int epi;                  // EPI_STORE (residual, next image), EPI_SWIGLU (image), EPI_QKV_ROPE
@@ -46,9 +47,14 @@ struct WideSplit {
     int split;
     size_t part_floats;
 };
-WideSplit wide_split(int M, int K, int N, int epi, int sm_count);
+WideSplit wide_split(int M, int K, int N, int w_terms, int epi, int sm_count);
 // One launch, or two: the product, and what follows it (see gemm_wide.cu).
 cudaError_t launch_gemm_wide(const WideArgs& a, int sm_count, cudaStream_t st, bool pdl, int* launches);
+// Q8_0 / Q4_0 blocks [n_rows][K / 32] -> tiles [ceil(N / 128)][K / 64][terms][128][64] of bf16 terms whose sum is the weight exactly (f16
+// scale times code: 19 bits, three terms; 15 bits, two).  Rows land at n_off + n, or interleaved 64 / 64 per block of 128 when
+// interleave_which is 0 (gate) or 1 (up).  K a multiple of 64.
+inline int wide_quant_terms(bool q4) { return q4 ? 2 : 3; }
+cudaError_t launch_wide_pack_quant(const uint8_t* blocks, int n_rows, int K, bool q4, uint16_t* dst, int n_off, int interleave_which, cudaStream_t st);
 // f32 rows -> activation image; folds an RMSNorm (weight norm_w) when norm_w is not null.
 cudaError_t launch_wide_pack(const float* x, int ldx, int M, int K, const float* norm_w, float eps, unsigned char* xp, cudaStream_t st, bool pdl);
 

@@ -69,3 +69,26 @@ def test_prompts_of_several_passes(hm, oracle):
     np.testing.assert_allclose(gk[0], ok, atol=5e-5)
     np.testing.assert_allclose(gv[0], ov, atol=5e-5)
     m.close()
+
+
+@pytest.mark.parametrize("gt,bias,norm", [(synth.GGML_Q8_0, False, False), (synth.GGML_Q4_0, False, False), (synth.GGML_Q8_0, True, False), (synth.GGML_Q4_0, False, True)])
+@pytest.mark.parametrize("n", [65, 128, 200])
+def test_quantised_prompts(hm, oracle, tmp_path, gt, bias, norm, n):
+    # whole prompt in one wide pass, and the same in passes of at most 64 rows: the weights are exact in both
+    cfg = synth.tiny_config(tie_word_embeddings=False, qkv_bias=bias, qk_norm=norm, head_dim=128 if norm else None, max_position_embeddings=256)
+    path = synth.write_gguf_model(str(tmp_path / "m.gguf"), cfg, 7, gt, norm_jitter=0.1)
+    om = oracle.OracleModel.from_gguf(path, max_seq_len=256)
+    m = hm.HfModel.load_gguf(path)
+    m.init_kv_cache(256)
+    ids = synth.prompt_ids(21, n + 1, cfg.vocab_size)
+    _, want = om.prefill(ids[:n])
+    tok, lg = m.prefill(ids[:n], want_logits=True)
+    ref = max(1.0, float(np.abs(want).max()))
+    assert float(np.abs(lg - want).max()) <= 3e-4 * ref  # the bound of the quantised batches
+    after = m.decode_step([int(ids[n])])[0][0]
+    m.reset_kv_cache()
+    for a in range(0, n, 60):
+        _, narrow = m.prefill(ids[a : min(n, a + 60)], want_logits=True)
+    assert float(np.abs(lg - narrow).max()) <= 3e-4 * ref
+    assert float(np.abs(after - m.decode_step([int(ids[n])])[0][0]).max()) <= 3e-4 * ref
+    m.close()
