@@ -9,7 +9,7 @@
 //     one accumulator.  Weights: 32 KB per 64-element k-block, shared by the three terms; activations: 16 KB per term.  Two rings
 //     (three weight slots, six term slots: 192 KB) so that a slot is refilled as soon as its own MMAs have read it.
 //   * the tensor core truncates when it adds to the accumulator, an error that grows with the length of the chain (2e-8 of the result
-//     per addition).  Accumulators therefore cover CHUNK k-blocks only; two of them (256 TMEM columns each) alternate,
+//     per addition at the result's magnitude).  Accumulators therefore cover CHUNK k-blocks only, the small terms of all of them first; two of them (256 TMEM columns each) alternate,
 //     and eight warps add the finished one to f32 registers (round to nearest) while the other is being filled.  A thread owns
 //     one row and 128 consecutive features, so that norms, rotation and gating need no exchange between threads.
 //   * Q8_0 and Q4_0 weights (f16 scale times code: 19 and 15 bits) come as three and two bf16 terms, exactly, and take the six and five
@@ -188,19 +188,27 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
             for (int u = blockIdx.x; u < a.units && ok; u += gridDim.x) {
                 const Unit t = unit_at(a, u);
                 const unsigned char* x0 = a.xp + (size_t)t.rb * rb_bytes;
+                auto load_x = [&](int kb, int term) {
+                    const uint32_t x = xi % X_SLOTS;
+                    if (xi >= X_SLOTS) ok = mb_wait(&sh.xempty[x], ((xi / X_SLOTS) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
+                    if (!ok) return;
+                    mb_expect_tx(&sh.xfull[x], X_SLOT);
+                    bulk_copy(xring + (size_t)x * X_SLOT, x0 + ((size_t)kb * 3 + term) * X_SLOT, X_SLOT, &sh.xfull[x]);
+                    ++xi;
+                };
                 for (int i = 0; i < (t.kb1 - t.kb0) * WT && ok; ++i, ++wi) {
                     const uint32_t s = wi % W_SLOTS;
                     if (wi >= W_SLOTS) ok = mb_wait(&sh.wempty[s], ((wi / W_SLOTS) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
                     if (!ok) break;
                     if (wi >= ahead) load_w(t, i, s);
-                    // the activation terms that this weight term is the first to meet
-                    const int w = WT - 1 - i % WT;
-                    for (int term = 2 - w; term >= (w == WT - 1 ? 0 : 2 - w); --term, ++xi) {
-                        const uint32_t x = xi % X_SLOTS;
-                        if (xi >= X_SLOTS) ok = mb_wait(&sh.xempty[x], ((xi / X_SLOTS) & 1u) ^ 1u, a.err_flag, &sh.abort_flag);
-                        if (!ok) break;
-                        mb_expect_tx(&sh.xfull[x], X_SLOT);
-                        bulk_copy(xring + (size_t)x * X_SLOT, x0 + ((size_t)(t.kb0 + i / WT) * 3 + term) * X_SLOT, X_SLOT, &sh.xfull[x]);
+                    const int kb = t.kb0 + i / WT;
+                    if (WT == 1) {  // the leading terms of a chunk behind the others of all its k-blocks
+                        for (int term = 2; term > 0 && ok; --term) load_x(kb, term);
+                        if (i % CHUNK<WT> == CHUNK<WT> - 1 || kb + 1 == t.kb1)
+                            for (int k = kb - i % CHUNK<WT>; k <= kb && ok; ++k) load_x(k, 0);
+                    } else {  // the activation terms that this weight term is the first to meet
+                        const int w = WT - 1 - i % WT;
+                        for (int term = 2 - w; term >= (w == WT - 1 ? 0 : 2 - w) && ok; --term) load_x(kb, term);
                     }
                 }
             }
@@ -219,7 +227,34 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     uint32_t more = 0;
                     const int ke = min(t.kb1, kc + CHUNK<WT>);
-                    for (int kb = kc; kb < ke && ok; ++kb, xi += 3) {
+                    if (WT == 1) {
+                        auto product = [&](uint32_t s) {  // the next activation term with weight slot s
+                            const uint32_t x = xi % X_SLOTS, wa = s32(wring + (size_t)s * W_SLOT), xa = s32(xring + (size_t)x * X_SLOT);
+                            ok = ok && mb_wait(&sh.xfull[x], (xi / X_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
+                            if (!ok) return;
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                            for (int ks = 0; ks < BK / 16; ++ks) {
+                                mma_f16(d, desc_sw128(xa + ks * 32), desc_sw128(wa + ks * 32), idesc, more);
+                                more = 1;
+                            }
+                            mma_commit(&sh.xempty[x]);
+                            ++xi;
+                        };
+                        // The small terms of the chunk while the accumulator is small, the leading ones last: only their additions
+                        // truncate at the magnitude of the result.
+                        for (int k = kc; k < ke && ok; ++k) {
+                            const uint32_t s = (wi + (k - kc)) % W_SLOTS;
+                            ok = mb_wait(&sh.wfull[s], ((wi + (k - kc)) / W_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
+                            product(s);
+                            product(s);
+                        }
+                        for (int k = kc; k < ke && ok; ++k, ++wi) {
+                            product(wi % W_SLOTS);
+                            if (ok) mma_commit(&sh.wempty[wi % W_SLOTS]);
+                        }
+                    }
+                    for (int kb = kc; WT > 1 && kb < ke && ok; ++kb, xi += 3) {
 #pragma unroll
                         for (int w = WT - 1; w >= 0; --w, ++wi) {
                             const uint32_t s = wi % W_SLOTS;
@@ -228,7 +263,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
 #pragma unroll
                             for (int term = 2 - w; term >= 0; --term) {  // small products first
                                 // place of the term among the three of this k-block: in the order of their first use
-                                const uint32_t xn = xi + (WT == 1 ? 2 - term : WT == 2 ? (term == 2 ? 2 : 1 - term) : term), x = xn % X_SLOTS;
+                                const uint32_t xn = xi + (WT == 2 ? (term == 2 ? 2 : 1 - term) : term), x = xn % X_SLOTS;
                                 if (w == WT - 1 || term == 2 - w) ok = ok && mb_wait(&sh.xfull[x], (xn / X_SLOTS) & 1u, a.err_flag, &sh.abort_flag);
                                 if (!ok) break;
                                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
