@@ -1163,8 +1163,8 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
     }
     const int QKV = qdim_ + 2 * kvdim_;
     const float eps = (float)cfg_.rms_norm_eps;
-    // more than 8 rows of a bf16 model: tensor-core projections with the epilogues as kernels of their own
-    const bool tall = use_tc_ && !quant_ && M > MAX_M;
+    // more than a few rows of a bf16 model: tensor-core projections
+    const bool tall = !quant_ && tall_rows(M);
     // Weight prefetch, decode passes of bf16 models: every kernel asks the L2 for the weights of the
     // kernel two launches ahead, so HBM keeps streaming while the short dependent kernels run.
     const bool pf = use_prefetch_ && !quant_ && !tall && only_class_ < 0;
@@ -1304,7 +1304,7 @@ int Engine::enqueue_logits(const float* x, int lm_rows, bool whole_pass, bool pa
     int rc;
     const int nslabs = (V_ + SLAB - 1) / SLAB;
     float* const lg = logits_ + lm_dst_row_ * V_;
-    const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows);
+    const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows) && !(lm_out_ && lm_rows <= MAX_M);  // (a head that stores into host memory streams)
     const bool slab_argmax = lm_head_.kind == HM_BF16;  // per-block argmax partials from the projection's epilogue
     const bool fold_argmax = slab_argmax && !lm_tall;    // the streaming kernel's last epilogue also produces the greedy token
     lm_folds_argmax_ = fold_argmax;

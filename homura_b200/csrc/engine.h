@@ -210,9 +210,12 @@ class Engine {
     int alloc_listed_cache(int batch, size_t n_pages);
     void free_listed_cache();
     void free_listed();
-    // Rows from which a pass's projections run on the tensor cores.  The grouped norms of listed designs cost the streaming kernel
-    // more per row, so theirs move over earlier.
-    bool tall_rows(int rows) const { return use_tc_ && rows > (spec_.listed() ? 4 : MAX_M); }
+    // Rows from which a pass's projections run on the tensor cores: the streaming kernel multiplies on the CUDA cores and is bound by
+    // them from five rows on.  Step of 5 / 8 sequences, streaming and tensor cores: 0.5 B 1.29 / 1.30 and 0.89 / 0.91 ms, 1.5 B 2.94 / 3.12
+    // and 1.42 / 1.51, 0.6 B 1.83 / 1.89 and 1.13 / 1.20; of 4: 0.70 and 0.89, 1.53 and 1.41, 1.01 and 1.10.  (The grouped norms of
+    // listed designs cost the streaming kernel more per row.)
+    static constexpr int FEW_ROWS = 4;
+    bool tall_rows(int rows) const { return use_tc_ && rows > FEW_ROWS; }
     int enqueue_listed_layer(int l, int M, const int32_t* row_pos, const int32_t* row_seq, int next_lm_rows, int* launches);
     // listed grouped-query attention, post-norms, mixtures of experts (engine_gqa.cu)
     int load_gqa_tensor(LayerW& w, const LayerSpec& s, const std::string& name, const std::string& rest, int dtype, const int64_t* shape, int ndim, const void* host, size_t nbytes);

@@ -556,6 +556,11 @@ __device__ void tc_epilogue(const TcArgs& a, float* tile, int m_lo, int m_hi, in
     }
 }
 
+// The k-blocks of a CTA take turns on several accumulators where few rows leave tensor memory for them: the tensor core truncates when it
+// adds, an error that grows with the length of the chain (K 1536 in one chain: 1.5e-6 of the result).
+__host__ __device__ __forceinline__ constexpr int acc_set(int mpad) { return mpad * 4; }  // columns of one: three terms, to a power of two
+static int tc_sets(int mpad, bool multi_wave) { return mpad == 16 ? (multi_wave ? 2 : 4) : mpad == 32 ? 2 : 1; }  // at most 256 columns; 128 where three CTAs share an SM
+
 // ---- the GEMM: warp 0 = bulk-copy producer, warp 1 = TMEM owner + MMA issuer, warps 2-5 = epilogue ----
 struct ExpertList {
     uint32_t mask[32];
@@ -563,7 +568,8 @@ struct ExpertList {
     int n;
 };
 
-template <bool CL, int V>
+// MS: several accumulators
+template <bool CL, int V, bool MS>
 __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) {
     constexpr bool X = V == 1 || V == 3;
     extern __shared__ __align__(1024) unsigned char dsm[];
@@ -704,7 +710,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = umma_idesc(TERMS * mpad);
+            const uint32_t idesc = umma_idesc(TERMS * mpad), set_cols = (uint32_t)acc_set(mpad), acc_end = tmem + (uint32_t)a.sets * set_cols;
+            const int sets = MS ? a.sets : 1;
+            uint32_t acc = tmem;
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % nst;
                 const uint32_t par = (i / nst) & 1u;
@@ -715,7 +723,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
                 const uint32_t xa = wa + W_TILE;
 #pragma unroll
                 for (int ks = 0; ks < BK / 16; ++ks)
-                    umma_f16(tmem, umma_desc_k_sw128(wa + ks * 32), umma_desc_k_sw128(xa + ks * 32), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+                    umma_f16(acc, umma_desc_k_sw128(wa + ks * 32), umma_desc_k_sw128(xa + ks * 32), idesc, (i >= sets || ks > 0) ? 1u : 0u);
+                if (MS) acc = acc + set_cols == acc_end ? tmem : acc + set_cols;
                 umma_commit(&sh.empty[s]);  // stage reusable once these MMAs have read it
             }
             umma_commit(&sh.acc_full);
@@ -750,24 +759,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs a) 
         const int lane_base = (warp & 3) * 32;  // a warp may only touch its own quarter of the TMEM lanes
         const int n_local = lane_base + lane;   // output feature within the CTA's 128
         if (acc_ok && nkb > 0) {
-            for (int c0 = 0; c0 < mpad; c0 += 16) {
+            const int sets = min(a.sets, nkb);
+            auto load = [&](uint32_t taddr, float (&v)[16], bool more) {
                 uint32_t r[TERMS][16];
 #pragma unroll
                 for (int t = 0; t < TERMS; ++t) {
-                    const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)(t * mpad + c0);
                     asm volatile(
                         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                         : "=r"(r[t][0]), "=r"(r[t][1]), "=r"(r[t][2]), "=r"(r[t][3]), "=r"(r[t][4]), "=r"(r[t][5]), "=r"(r[t][6]), "=r"(r[t][7]), "=r"(r[t][8]), "=r"(r[t][9]),
                           "=r"(r[t][10]), "=r"(r[t][11]), "=r"(r[t][12]), "=r"(r[t][13]), "=r"(r[t][14]), "=r"(r[t][15])
-                        : "r"(taddr));
+                        : "r"(taddr + (uint32_t)(t * mpad)));
                 }
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     // small terms first: lo + mid, then + hi
-                    const float v = (__uint_as_float(r[2][j]) + __uint_as_float(r[1][j])) + __uint_as_float(r[0][j]);
-                    out_tile[(c0 + j) * BM + n_local] = scale_rows ? v * sh.inv[c0 + j] : v;
+                    const float x = (__uint_as_float(r[2][j]) + __uint_as_float(r[1][j])) + __uint_as_float(r[0][j]);
+                    v[j] = more ? v[j] + x : x;
                 }
+            };
+            for (int c0 = 0; c0 < mpad; c0 += 16) {
+                float v[16];
+                const uint32_t taddr = tmem + ((uint32_t)lane_base << 16) + (uint32_t)c0;
+                load(taddr, v, false);
+                if (MS)
+                    for (int set = 1; set < sets; ++set) load(taddr + (uint32_t)(set * acc_set(mpad)), v, true);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) out_tile[(c0 + j) * BM + n_local] = scale_rows ? v[j] * sh.inv[c0 + j] : v[j];
             }
         } else {
             for (int mm = 0; mm < mpad; ++mm) out_tile[mm * BM + n_local] = 0.f;
@@ -890,7 +908,7 @@ cudaError_t launch_tc_pack_gnorm(const float* x, int ldx, int M, int K, const fl
     return cudaLaunchKernelEx(&cfg, tc_pack_gnorm_kernel, x, ldx, M, tc_mpad(M), K, Kp, norm_w, eps, gn, (unsigned char*)xp);
 }
 
-template <int V>
+template <int V, bool MS>
 static cudaError_t launch_gemm_tc_v(const TcArgs& a_in, cudaStream_t st, bool pdl) {
     TcArgs a = a_in;
     if (a.M < 1 || a.M > MR || a.Kp % BK != 0 || !a.xp) return cudaErrorInvalidValue;
@@ -909,12 +927,13 @@ static cudaError_t launch_gemm_tc_v(const TcArgs& a_in, cudaStream_t st, bool pd
     }
     const bool multi_wave = (long)busy * (a.ksplit > 1 ? a.ksplit : 1) > sms;
     a.nstage = tc_nstage(a.mpad, multi_wave);
-    a.tmem_cols = a.mpad == 16 ? 64 : a.mpad == 32 ? 128 : 256;  // power of two >= 3 * mpad
+    a.sets = MS ? tc_sets(a.mpad, multi_wave) : 1;
+    a.tmem_cols = a.sets * acc_set(a.mpad);
     const bool cl = a.ksplit > 1;
     const size_t smem = tc_smem_for(a.mpad, multi_wave) + (cl ? tc_recv_bytes(a.M, a.ksplit) : 0);
     {
         const size_t mx = (tc_smem_for(64, false) > tc_smem_for(32, false) ? tc_smem_for(64, false) : tc_smem_for(32, false)) + (cl ? (size_t)(MR + 16) * BM * 4 : 0);
-        cudaError_t e = cl ? ensure_dyn_smem(gemm_tc_kernel<true, V>, mx) : ensure_dyn_smem(gemm_tc_kernel<false, V>, mx);
+        cudaError_t e = cl ? ensure_dyn_smem(gemm_tc_kernel<true, V, MS>, mx) : ensure_dyn_smem(gemm_tc_kernel<false, V, MS>, mx);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -932,7 +951,7 @@ static cudaError_t launch_gemm_tc_v(const TcArgs& a_in, cudaStream_t st, bool pd
     if (cl) {
         if (a.ksplit > 16) return cudaErrorInvalidValue;
         if (a.ksplit > 8) {  // clusters of 9..16 CTAs are allowed on request
-            cudaError_t e = ensure_nonportable_clusters(gemm_tc_kernel<true, V>);
+            cudaError_t e = ensure_nonportable_clusters(gemm_tc_kernel<true, V, MS>);
             if (e != cudaSuccess) return e;
         }
         at[n].id = cudaLaunchAttributeClusterDimension;
@@ -943,14 +962,16 @@ static cudaError_t launch_gemm_tc_v(const TcArgs& a_in, cudaStream_t st, bool pd
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return cl ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true, V>, a) : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, V>, a);
+    return cl ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true, V, MS>, a) : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false, V, MS>, a);
 }
 
 cudaError_t launch_gemm_tc(const TcArgs& a, cudaStream_t st, bool pdl) {
     const bool x = a.group_blocks || a.out_scale || a.split_xp || a.epi == EPI_GATE || a.epi == EPI_SQRELU;
-    if (a.ex.n) return launch_gemm_tc_v<2>(a, st, pdl);
-    if (a.turn.turns || a.softcap > 0.f || a.epi == EPI_GLU || (a.epi == EPI_GATE && a.gate_per > 1)) return launch_gemm_tc_v<3>(a, st, pdl);
-    return x ? launch_gemm_tc_v<1>(a, st, pdl) : launch_gemm_tc_v<0>(a, st, pdl);
+    const bool few = tc_mpad(a.M) < MR;  // (mixtures of experts, rotations and capped logits keep one accumulator)
+    if (a.ex.n) return launch_gemm_tc_v<2, false>(a, st, pdl);
+    if (a.turn.turns || a.softcap > 0.f || a.epi == EPI_GLU || (a.epi == EPI_GATE && a.gate_per > 1)) return launch_gemm_tc_v<3, false>(a, st, pdl);
+    if (few) return x ? launch_gemm_tc_v<1, true>(a, st, pdl) : launch_gemm_tc_v<0, true>(a, st, pdl);
+    return x ? launch_gemm_tc_v<1, false>(a, st, pdl) : launch_gemm_tc_v<0, false>(a, st, pdl);
 }
 
 // ---- weight packing: [N][K] (HF [out,in]) or [K][N] bf16 -> swizzled K-major tiles ----------

@@ -34,7 +34,7 @@ struct TcArgs {
     int M;              // activation rows, 1..64
     int ksplit;         // CTAs per cluster sharing one n-block (1 = no split, at most 16)
     const unsigned char* xp;  // activations packed by launch_tc_pack_x (tc_xpack_bytes(M, K) bytes)
-    int mpad, nstage, tmem_cols;  // filled in by launch_gemm_tc
+    int mpad, nstage, tmem_cols, sets;  // filled in by launch_gemm_tc
     int epi;                 // EPI_STORE (bias, residual), EPI_SWIGLU, EPI_LOGITS or EPI_QKV_ROPE: as in GemvArgs
     const float* bias;       // optional [N]
     const float* resid;      // optional [M][ldy], added as resid + y
