@@ -1514,7 +1514,7 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
     HM_CUDA(cudaStreamSynchronize(stream_));
     int rc = check_device_error();
     if (rc) return rc;
-    if (logits && land != logits) std::memcpy(logits, land, (size_t)V_ * 4);
+    if (logits && land != logits) copy_out(logits, land, (size_t)V_ * 4);
     if (first_token) *first_token = *tok_pin;
     len_[seq] = len0 + n;
     gen_start_[seq] = len0 + n;  // what follows this prompt is "generated" for the penalties (src/generate.rs:150-152)
@@ -1552,7 +1552,7 @@ int Engine::decode_step(const uint32_t* tokens, float* logits, uint32_t* next_to
         int erc = check_device_error();
         if (erc) return erc;
     }
-    if (logits && land != logits) std::memcpy(logits, land, (size_t)batch_ * V_ * 4);
+    if (logits && land != logits) copy_out(logits, land, (size_t)batch_ * V_ * 4);
     if (next_tokens) std::memcpy(next_tokens, pin_u32_ + batch_, (size_t)batch_ * 4);
     for (int b = 0; b < batch_; ++b) len_[b] += 1;
     return HM_OK;
@@ -1888,7 +1888,7 @@ int Engine::decode_step_sampled(const uint32_t* tokens, const hm_sampling* sp, u
     HM_CUDA(cudaStreamSynchronize(stream_));
     rc = check_device_error();
     if (rc) return rc;
-    if (logits && land != logits) std::memcpy(logits, land, B * V_ * 4);
+    if (logits && land != logits) copy_out(logits, land, B * V_ * 4);
     std::memcpy(rng_state, pin_rng, B * 8);
     std::vector<float> row;
     std::vector<uint32_t> gen;
