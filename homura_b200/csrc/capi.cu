@@ -794,7 +794,8 @@ int hm_gemm_bf16_tc(const float* x, const void* w_tc, int M, int K, int N, int k
     if (!sg.ok(get_scratch((tc_xpack_bytes(M, K) + 3) / 4, 1, &xp, &unused))) return sg.finish(cudaSuccess);
     a.xp = (const unsigned char*)xp;
     cudaError_t ce = launch_tc_pack_x(xd, K, M, K, nullptr, 0.f, xp, st, false);
-    if (ce == cudaSuccess) ce = launch_gemm_tc(a, st, false);
+    // the product may start its weights while the packing launch runs, which is itself ordered behind everything before it
+    if (ce == cudaSuccess) ce = launch_gemm_tc(a, st, true);
     const bool synced = sg.staged();
     const int rc = sg.finish(ce);
     if (rc != HM_OK) return rc;
