@@ -634,7 +634,10 @@ __device__ __forceinline__ void split3_pack(float x, float y, uint32_t (&t)[3]) 
 }
 __host__ __device__ constexpr size_t st_q_bytes(int hd) { return 3 * (size_t)(hd / 16) * 32 * 8 > (size_t)G_MAX * hd * 4 ? 3 * (size_t)(hd / 16) * 32 * 8 : (size_t)G_MAX * hd * 4; }
 
-template <int HD, bool BF16, bool CL>
+// GH: query heads per KV head on f32 pages.  The loops of a page are unrolled over the heads, and heads that may or may not be there cost a
+// test each, in loops that the issue rate bounds.  One variant for up to eight heads, and now: 8 sequences x 16384 tokens, 2 heads per KV head
+// of 128: 289 -> 173 us (6.2 TB/s); 6 heads of 128: 118 -> 78; 7 heads of 64: 51.7 -> 43.3; 64 x 500, 6 of 128: 34.7 -> 23.6.
+template <int HD, bool BF16, bool CL, int GH>
 __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnArgs a) {
     using ST = StTile<HD, BF16>;
     using T = typename std::conditional<BF16, uint16_t, float>::type;
@@ -739,9 +742,9 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
 #pragma unroll
     for (int mt = 0; mt < (BF16 ? HD / 16 : 1); ++mt) to[mt][0] = to[mt][1] = to[mt][2] = to[mt][3] = 0.f;
     // per-warp running softmax state of every head; the page loop leaves warps with different maxima
-    float run_m[G_MAX], run_l[G_MAX], acc[G_MAX][EPL];
+    float run_m[GH], run_l[GH], acc[GH][EPL];
 #pragma unroll
-    for (int jj = 0; jj < G_MAX; ++jj) {
+    for (int jj = 0; jj < GH; ++jj) {
         run_m[jj] = -INFINITY;
         run_l[jj] = 0.f;
 #pragma unroll
@@ -868,29 +871,29 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
             const int p = p0 + i;
             // ---- scores of the 16 tokens against all g heads: lane = (token, half of hd) ----
             // packed f32x2 FMAs: even and odd elements of a chunk accumulate in the two halves of a pair
-            float2 sc2[G_MAX];
+            float2 sc2[GH];
 #pragma unroll
-            for (int jj = 0; jj < G_MAX; ++jj) sc2[jj] = make_float2(0.f, 0.f);
+            for (int jj = 0; jj < GH; ++jj) sc2[jj] = make_float2(0.f, 0.f);
 #pragma unroll 4
             for (int c = 0; c < NCH; ++c) {
                 const float4 k4 = ld_chunk4<BF16>(kt, (((hf * NCH + c) << 4) + t) << 2);  // chunk-major K tile
 #pragma unroll
-                for (int jj = 0; jj < G_MAX; ++jj) {
-                    if (jj < g) {
+                for (int jj = 0; jj < GH; ++jj) {
+                    if (BF16 ? jj < g : true) {
                         const float4 q4 = *reinterpret_cast<const float4*>(q_s + jj * HD + (c * 2 + hf) * 4);
                         sc2[jj] = __ffma2_rn(make_float2(q4.x, q4.y), make_float2(k4.x, k4.y), sc2[jj]);
                         sc2[jj] = __ffma2_rn(make_float2(q4.z, q4.w), make_float2(k4.z, k4.w), sc2[jj]);
                     }
                 }
             }
-            float sc[G_MAX];
+            float sc[GH];
 #pragma unroll
-            for (int jj = 0; jj < G_MAX; ++jj) sc[jj] = sc2[jj].x + sc2[jj].y;
+            for (int jj = 0; jj < GH; ++jj) sc[jj] = sc2[jj].x + sc2[jj].y;
             const bool valid = (p * PT + t) < kvlen;
-            float corr[G_MAX];
+            float corr[GH];
 #pragma unroll
-            for (int jj = 0; jj < G_MAX; ++jj) {
-                if (jj < g) {
+            for (int jj = 0; jj < GH; ++jj) {
+                if (BF16 ? jj < g : true) {
                     float sv = sc[jj] + __shfl_xor_sync(0xffffffffu, sc[jj], 16);
                     sv = valid ? sv * a.scale : -INFINITY;
                     float mx = sv;
@@ -910,9 +913,9 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
             __syncwarp();
             // ---- p . v: lane owns EPL output dims of every head; a V row is read once for all heads ----
 #pragma unroll
-            for (int jj = 0; jj < G_MAX; ++jj)
+            for (int jj = 0; jj < GH; ++jj)
 #pragma unroll
-                for (int e = 0; e < EPL; ++e) acc[jj][e] *= (jj < g) ? corr[jj] : 1.f;
+                for (int e = 0; e < EPL; ++e) acc[jj][e] *= corr[jj];
 #pragma unroll
             for (int t4 = 0; t4 < PT; t4 += 4) {
                 float vv[4][EPL];
@@ -929,8 +932,8 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
                     }
                 }
 #pragma unroll
-                for (int jj = 0; jj < G_MAX; ++jj) {
-                    if (jj < g) {
+                for (int jj = 0; jj < GH; ++jj) {
+                    if (BF16 ? jj < g : true) {
                         const float4 p4 = *reinterpret_cast<const float4*>(pw + jj * PT + t4);  // broadcast
 #pragma unroll
                         for (int e = 0; e < EPL; ++e) {
@@ -952,7 +955,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             const int jj = tig * 2 + hh;
-            if (jj < g) {
+            if (BF16 ? jj < g : true) {
                 const int w = warp * g + jj;
                 if (gid == 0) {
                     w_ml[w * 2 + 0] = tm[hh];
@@ -968,8 +971,8 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
     } else if (warp < ST::CW) {
         // publish this warp's state: slot = warp, entry (warp * g + head)
 #pragma unroll
-        for (int jj = 0; jj < G_MAX; ++jj) {
-            if (jj < g) {
+        for (int jj = 0; jj < GH; ++jj) {
+            if (BF16 ? jj < g : true) {
                 const int w = warp * g + jj;
                 if (lane == 0) {
                     w_ml[w * 2 + 0] = run_m[jj];
@@ -996,7 +999,7 @@ size_t smem_bytes(int g, int slots, int nslots) {
     return sizeof(float) * ((size_t)G_MAX * HD + (size_t)nslots * TL::SLOT_FLOATS + ATT_WARPS * PT + ATT_WARPS * 2 + ATT_WARPS * HD + (size_t)slots * g * (HD + 2));
 }
 
-template <int HD, bool BF16, bool CL>
+template <int HD, bool BF16, bool CL, int GH>
 cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     const int g = a.heads / a.kv_heads;
     const int pages_per_cta = (a.max_pages + a.nsplit - 1) / a.nsplit;
@@ -1021,8 +1024,8 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     const size_t smem = stream ? stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, stages) : smem_bytes<HD, BF16>(g, slots, pick_nslots<HD, BF16>(g, a.early_pages, a.max_pages, a.nsplit));
     // per device, and only ever raised: launches captured in a graph must stay valid after later calls
     {
-        cudaError_t e = stream ? ensure_dyn_smem(attn_stream_kernel<HD, BF16, CL>, smem) : ensure_dyn_smem(attn_decode_kernel<HD, BF16, CL>, smem);
-        if (e == cudaSuccess && CL && a.nsplit > 8) e = stream ? ensure_nonportable_clusters(attn_stream_kernel<HD, BF16, CL>) : ensure_nonportable_clusters(attn_decode_kernel<HD, BF16, CL>);
+        cudaError_t e = stream ? ensure_dyn_smem(attn_stream_kernel<HD, BF16, CL, GH>, smem) : ensure_dyn_smem(attn_decode_kernel<HD, BF16, CL>, smem);
+        if (e == cudaSuccess && CL && a.nsplit > 8) e = stream ? ensure_nonportable_clusters(attn_stream_kernel<HD, BF16, CL, GH>) : ensure_nonportable_clusters(attn_decode_kernel<HD, BF16, CL>);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -1046,16 +1049,33 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return stream ? cudaLaunchKernelEx(&cfg, attn_stream_kernel<HD, BF16, CL>, a2) : cudaLaunchKernelEx(&cfg, attn_decode_kernel<HD, BF16, CL>, a2);
+    return stream ? cudaLaunchKernelEx(&cfg, attn_stream_kernel<HD, BF16, CL, GH>, a2) : cudaLaunchKernelEx(&cfg, attn_decode_kernel<HD, BF16, CL>, a2);
+}
+
+template <int HD, bool BF16, bool CL>
+cudaError_t launch_g(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
+    const int g = a.heads / a.kv_heads;
+    if constexpr (!BF16) {
+        switch (g) {
+            case 1: return launch_tc<HD, BF16, CL, 1>(a, M, st, pdl);
+            case 2: return launch_tc<HD, BF16, CL, 2>(a, M, st, pdl);
+            case 3: return launch_tc<HD, BF16, CL, 3>(a, M, st, pdl);
+            case 4: return launch_tc<HD, BF16, CL, 4>(a, M, st, pdl);
+            case 5: return launch_tc<HD, BF16, CL, 5>(a, M, st, pdl);
+            case 6: return launch_tc<HD, BF16, CL, 6>(a, M, st, pdl);
+            case 7: return launch_tc<HD, BF16, CL, 7>(a, M, st, pdl);
+        }
+    }
+    return launch_tc<HD, BF16, CL, G_MAX>(a, M, st, pdl);
 }
 
 template <int HD, bool BF16>
 cudaError_t launch_t(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     if (a.cluster) {
         if (a.nsplit < 1 || a.nsplit > 16) return cudaErrorInvalidValue;
-        return launch_tc<HD, BF16, true>(a, M, st, pdl);
+        return launch_g<HD, BF16, true>(a, M, st, pdl);
     }
-    return launch_tc<HD, BF16, false>(a, M, st, pdl);
+    return launch_g<HD, BF16, false>(a, M, st, pdl);
 }
 
 }  // namespace

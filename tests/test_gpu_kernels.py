@@ -329,3 +329,16 @@ def test_kquant_gemv_matches_oracle(hm, oracle, kind, dt, gt, M, K, N):
     assert rel_err(got, want) < 1e-5
     if K == 256:  # one super-block per row: no reordering at all
         np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("heads,kvh,hd", [(g * kvh, kvh, hd) for g, kvh, hd in [(1, 4, 128), (2, 2, 64), (3, 2, 128), (4, 2, 128), (5, 1, 64), (6, 1, 64), (7, 1, 128), (8, 1, 128)]])
+def test_attention_of_every_number_of_heads_per_kv_head(hm, oracle, heads, kvh, hd):
+    # f32 pages: the streaming kernel has variants by the number of query heads per KV head; tolerance as above
+    rng = np.random.default_rng(heads + hd)
+    lens = [2100, 16, 1025]
+    kd, vd, perm, max_pages, ks, vs = _paged(rng, len(lens), kvh, hd, lens, False, hm)
+    q = rng.standard_normal((len(lens), heads, hd), dtype=np.float32)
+    got = hm.attn_decode_paged(q, kd, vd, hm.DType.F32, perm, lens, heads, kvh, hd, max_pages)
+    for b, L in enumerate(lens):
+        want = oracle.gqa_attention(q[b : b + 1], ks[b], vs[b], np.zeros((1, L), np.float32), heads, kvh)
+        np.testing.assert_allclose(got[b], want[0], rtol=0, atol=3e-6 * max(1.0, float(np.abs(want).max())))
