@@ -234,7 +234,7 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
         if (ce == cudaSuccess) ce = launch_split_blocks((const uint8_t*)tmp, n_part, K, q4, n_off, interleave_which, L.scales, L.codes, stream_, rope_hd);
         quant_ = true;
         // a second copy for prompts (4 or 6 bytes per weight); without the memory for it prompts run in passes of 64 rows
-        if (ce == cudaSuccess && use_tc_ && &L != &lm_head_ && K % 64 == 0) {
+        if (ce == cudaSuccess && use_tc_ && &L != &lm_head_ && K % 64 == 0 && wide_copies_fit(wide_quant_terms(q4))) {
             if (!L.wide && L.loaded_parts == 0) {
                 L.wide_terms = wide_quant_terms(q4);
                 const size_t bytes = tc_packed_elems(K, N_total) * 2 * L.wide_terms;
@@ -646,6 +646,7 @@ int Engine::kv_free() {
     };
     for (void*& p : k_pool_) fr(p);
     for (void*& p : v_pool_) fr(p);
+    free_wide();
     k_pool_.clear();
     v_pool_.clear();
     free_listed_cache();
@@ -1177,7 +1178,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
     };
     constexpr size_t LM_PF = 24u << 20;  // the LM head does not fit the L2: only its first 2 x 24 MB are fetched early
     int rc;
-    // passes of 9..64 rows: the attention output and the SwiGLU output go straight into the packed
+    // passes of 5..64 rows: the attention output and the SwiGLU output go straight into the packed
     // activation tiles of the next tensor-core GEMM (no packing launch in between) ...
     const bool direct_pack = tall && M <= TC_ROWS && qdim_ % 64 == 0 && I_ % 64 == 0;
     // ... and so does the hidden state after the O and down projections, whose RMSNorm is split between the

@@ -197,6 +197,7 @@ class Engine {
     AttnArgs attn_args(int l, int M, const float* q, const int32_t* row_pos, const int32_t* row_seq) const;
     // passes over many rows (engine_wide.cu)
     bool wide_fits() const;
+    bool wide_copies_fit(int terms) const;
     bool ensure_wide(int rows);
     int plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan);
     int enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches);

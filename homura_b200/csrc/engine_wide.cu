@@ -26,6 +26,18 @@ bool Engine::wide_fits() const {
     return true;
 }
 
+// Whether all projections of a quantised model may be held as bf16 terms as well: in at most an eighth of the GPU's memory (22 GB: models
+// of up to 3.8 B weights in Q8_0), so that models near its limits keep it for their caches.
+bool Engine::wide_copies_fit(int terms) const {
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const double weights = (double)L_ * ((double)H_ * (2.0 * qdim_ + 2.0 * kvdim_) + 3.0 * H_ * I_);
+    return weights * 2 * terms <= (double)total / 8;
+}
+
 void Engine::free_wide() {
     for (void* p : {(void*)wide_.h, (void*)wide_.q, (void*)wide_.ss, (void*)wide_.ss2, (void*)wide_.x, (void*)wide_.x2, (void*)wide_.att, (void*)wide_.act, (void*)wide_.part, (void*)wide_.staged, (void*)wide_.tables})
         if (p) cudaFree(p);
