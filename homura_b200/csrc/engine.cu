@@ -185,7 +185,7 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
         }
         if (ce == cudaSuccess) ce = launch_pack_slabs_from_nk((const uint16_t*)tmp, n_part, K, L.slabs, n_off, interleave_which, stream_);
         if (use_tc_ && ce == cudaSuccess) {
-            // second copy for passes over more than 8 rows (same 64 + 64 gate/up interleave per 128 features)
+            // second copy for passes over more than four rows (same 64 + 64 gate/up interleave per 128 features)
             if (!L.tc) {
                 const size_t bytes = tc_packed_elems(K, N_total) * 2;
                 ce = cudaMalloc(&L.tc, bytes);
@@ -468,7 +468,7 @@ int Engine::ensure_scratch(int rows) {
     HM_CUDA(re(&amax_val_, (size_t)cap * nslabs_v));
     HM_CUDA(re(&amax_idx_, (size_t)cap * nslabs_v));
     if (!tall && use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc) {
-        // a GGUF model whose LM head is the bf16 embedding: passes over more than 8 rows run that one projection on the tensor cores
+        // a GGUF model whose LM head is the bf16 embedding: passes over more than four rows run that one projection on the tensor cores
         xpack_bytes_ = tc_xpack_bytes(TC_ROWS, H_);
         HM_CUDA(re(&xpack_, xpack_bytes_));
     }

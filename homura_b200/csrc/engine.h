@@ -30,7 +30,7 @@ struct LinearW {
     int K = 0, N = 0;        // N = output count of the (possibly fused) projection
     int kind = -1;           // HM_BF16 (slab layout) | HM_Q8_0 | HM_Q4_0 (split scales + codes)
     uint16_t* slabs = nullptr;
-    uint16_t* tc = nullptr;  // second copy in the tensor-core tile layout (gemm_tc.h), used for passes over more than 8 rows
+    uint16_t* tc = nullptr;  // second copy in the tensor-core tile layout (gemm_tc.h), used for passes over more than four rows
     uint16_t* wide = nullptr;  // Q8_0 / Q4_0: the weights as bf16 terms (gemm_wide.h), for prompts of more than 64 rows
     int wide_terms = 0;
     uint16_t* scales = nullptr;
@@ -308,7 +308,7 @@ class Engine {
     bool use_prefetch_ = true;  // decode kernels pull the weights of the kernel two launches ahead into the L2
     const void* pf_ptr_ = nullptr;  // prefetch target handed to the next projection launch
     unsigned long long pf_bytes_ = 0;
-    bool use_tc_ = true;  // bf16 models: passes over more than 8 rows run the tcgen05 GEMM (HM_NO_TC=1: 8-row groups of the streaming kernel)
+    bool use_tc_ = true;  // bf16 models: passes over more than four rows run the tcgen05 GEMM (HM_NO_TC=1: 8-row groups of the streaming kernel)
     cudaStream_t stream_ = nullptr;
 
     // weights

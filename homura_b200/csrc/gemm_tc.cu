@@ -1,4 +1,4 @@
-// Skinny tensor-core GEMM for 9..64 activation rows: y[M,N] = x[M,K] @ W with bf16 weights, f32
+// Skinny tensor-core GEMM for 5..64 activation rows: y[M,N] = x[M,K] @ W with bf16 weights, f32
 // activations and f32 accumulation -- Homura's mixed matmul (src/graph_builder/emit_linalg.rs:
 // 1928-2008, 2224-2307) where the contraction is dense enough for the 5th-generation tensor cores
 // (batched decode, prefill chunks).
