@@ -1305,7 +1305,9 @@ int Engine::enqueue_logits(const float* x, int lm_rows, bool whole_pass, bool pa
     int rc;
     const int nslabs = (V_ + SLAB - 1) / SLAB;
     float* const lg = logits_ + lm_dst_row_ * V_;
-    const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows) && !(lm_out_ && lm_rows <= MAX_M);  // (a head that stores into host memory streams)
+    // A head that stores into host memory streams.  The listed designs' logits know no such exception: they decide by the rows alone.
+    const bool to_host = lm_out_ && !spec_.listed() && lm_rows <= MAX_M;
+    const bool lm_tall = use_tc_ && lm_head_.kind == HM_BF16 && lm_head_.tc && tall_rows(lm_rows) && !to_host;
     const bool slab_argmax = lm_head_.kind == HM_BF16;  // per-block argmax partials from the projection's epilogue
     const bool fold_argmax = slab_argmax && !lm_tall;    // the streaming kernel's last epilogue also produces the greedy token
     lm_folds_argmax_ = fold_argmax;
