@@ -88,8 +88,7 @@ __device__ __forceinline__ void unpack_store(float* o, const uint4& v) {
 // activation tiles of the O-projection's tensor-core GEMM.
 template <int HD>
 __device__ __forceinline__ void store_out(const AttnArgs& a, int m, int head, int d, float v) {
-    const int r = m + a.xp_row0;
-    if (a.xp_out) tc_xpack_store(a.xp_out + (size_t)(r >> 7) * a.xp_block, a.xp_mpad, r & 127, head * HD + d, v);
+    if (a.xp_out) tc_xpack_store(a.xp_out, a.xp_mpad, m, head * HD + d, v);
     else a.out[(size_t)m * a.heads * HD + head * HD + d] = v;
 }
 

@@ -495,8 +495,6 @@ struct AttnArgs {
     unsigned long long pf_bytes;
     unsigned char* xp_out;  // optional: write the output as packed tensor-core activations (tc_xpack_store) instead of `out`
     int xp_mpad;
-    size_t xp_block;        // an image of several row blocks of xp_mpad rows (gemm_wide.h): bytes from one to the next,
-    int xp_row0;            // and where row 0 of this launch belongs
     int early_pages;     // >= 1: every row is its own sequence (decode), so the pages below the one of the new token may be read before the dependency wait;
                          // 2: and every page of a split gets its own shared-memory slot (small launches, where latency counts and occupancy does not)
     int stream_pages;    // > 0: long contexts may use the bulk-copy ring variant (pages per CTA decided from max_pages / nsplit)

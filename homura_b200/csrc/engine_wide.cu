@@ -213,17 +213,19 @@ int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_
             ce = launch_attn_prefill(a, stream_, pdl_, launches);
             if (ce != cudaSuccess) return cuda_fail(ce, "prompt attention");
         }
+        // A launch writes the image from its own row 0 on: it stays within a block of 128 rows and starts on a multiple of eight, with which
+        // the image's swizzle repeats (the up to seven rows in front, of the prompt attention above, are done again).  An offset within the
+        // image as arguments of the decode kernel cost it four registers, and the steps of the 1.5 B stack 8 us per layer (f32 pages: 1.25 -> 1.49 ms).
         for (const WidePass::Range& r : p.singles)
-            for (int r0 = r.row0; r0 < r.row0 + r.rows; r0 += scratch_rows_) {
-                const int n = std::min(scratch_rows_, r.row0 + r.rows - r0);
+            for (int r0 = r.row0 & ~7, end = r.row0 + r.rows; r0 < end;) {
+                const int in_block = r0 % WIDE_BLOCK, n = std::min(std::min(scratch_rows_, end - r0), WIDE_BLOCK - in_block);
                 AttnArgs at = attn_args(l, n, wide_.q + (size_t)r0 * qdim_, row_pos + r0, row_seq + r0);
-                at.xp_out = wide_.att;
+                at.xp_out = wide_.att + (size_t)(r0 / WIDE_BLOCK) * wide_block_bytes(qdim_) + (size_t)in_block * 128;
                 at.xp_mpad = WIDE_BLOCK;
-                at.xp_block = wide_block_bytes(qdim_);
-                at.xp_row0 = r0;
                 ce = launch_attn_decode(at, n, kv_bf16_, stream_, pdl_);
                 if (ce != cudaSuccess) return cuda_fail(ce, "attention launch");
                 ++*launches;
+                r0 += n;
             }
         WideArgs o{};
         o.resid = wide_.h;

@@ -35,16 +35,18 @@ def test_prompts_at_the_edges_of_the_tiles(hm, oracle, name, kv, n):
 
 
 @pytest.mark.parametrize("name", ["qwen2", "qwen3"])
-def test_mixed_runs_of_any_length(hm, oracle, name):
-    # one token, 7 (row by row), 8 and 130 rows (tiles) in one batch, behind contexts of their own; every row's logits
+# One token, 7 (row by row), 8 and 130 rows (tiles) in one batch; short runs from row 107 on, which is no multiple of eight, over row 128,
+# and at the end.  All behind contexts of their own; every row's logits.
+@pytest.mark.parametrize("before,rows", [([40, 0, 17, 64, 3], [1, 7, 8, 130, 1]), ([0, 9, 5, 33, 16, 1, 70, 2], [107, 7, 7, 7, 1, 3, 20, 5])])
+def test_mixed_runs_of_any_length(hm, oracle, name, before, rows):
     cfg, d = make_hf(name, max_position_embeddings=256)
     m = hm.HfModel.load(d)
-    m.init_kv_cache(256, batch=5, pool_tokens=5 * 256)
-    before, rows = [40, 0, 17, 64, 3], [1, 7, 8, 130, 1]
+    n = len(rows)
+    m.init_kv_cache(256, batch=n, pool_tokens=n * 256)
     ids = [synth.prompt_ids(50 + i, b + r + 1, cfg.vocab_size) for i, (b, r) in enumerate(zip(before, rows))]
     want = [oracle.OracleModel.from_hf_dir(d, max_seq_len=256).forward_all(t) for t in ids]
-    m.step([(i, ids[i][: before[i]], []) for i in range(5) if before[i]], want_logits=False)
-    got, greedy, hidden = m.step([(i, ids[i][before[i] : before[i] + rows[i]], np.arange(rows[i])) for i in range(5)], want_logits=True, want_greedy=True, want_hidden=True)
+    m.step([(i, ids[i][: before[i]], []) for i in range(n) if before[i]], want_logits=False)
+    got, greedy, hidden = m.step([(i, ids[i][before[i] : before[i] + rows[i]], np.arange(rows[i])) for i in range(n)], want_logits=True, want_greedy=True, want_hidden=True)
     ref = np.concatenate([w[b : b + r] for w, b, r in zip(want, before, rows)])
     assert_logits_close(got, ref)
     assert greedy.tolist() == [oracle.argmax(r) for r in ref]
