@@ -347,7 +347,8 @@ class Engine {
     // passes over many rows: activations, activation images (gemm_wide.h), partial tiles, staged keys and values, tables
     struct Wide {
         int cap = 0;                     // rows
-        float *h = nullptr, *q = nullptr, *ss = nullptr, *ss2 = nullptr;
+        float *h = nullptr, *q = nullptr;
+        double *ss = nullptr, *ss2 = nullptr;
         unsigned char *x = nullptr, *x2 = nullptr, *att = nullptr, *act = nullptr;
         float* part = nullptr;
         unsigned char* staged = nullptr;

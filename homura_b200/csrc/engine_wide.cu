@@ -157,7 +157,7 @@ int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_
     const float eps = (float)cfg_.rms_norm_eps;
     cudaError_t ce = launch_embed_gather(embed_, embed_dtype_ == HM_BF16 ? 1 : 0, tokens, M, H_, V_, wide_.h, err_flag_, stream_, pdl_);
     if (ce != cudaSuccess) return cuda_fail(ce, "embed_gather");
-    ce = launch_wide_pack(wide_.h, H_, M, H_, layers_[0].in_ln, eps, wide_.x, stream_, pdl_);
+    ce = launch_wide_pack(wide_.h, H_, M, H_, layers_[0].in_ln, eps, quant_, wide_.x, stream_, pdl_);
     if (ce != cudaSuccess) return cuda_fail(ce, "activation pack");
     *launches += 2;
     for (int l = 0; l < L_; ++l) {

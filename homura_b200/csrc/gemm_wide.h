@@ -27,8 +27,9 @@ struct WideArgs {
     int ldy;
     unsigned char* xp_out;    // EPI_SWIGLU: image of the activations; EPI_STORE, optional: image of y * next_norm_w
     const float* next_norm_w;
-    float* ss_out;            // EPI_STORE with xp_out: [N / 128][ss_ld] sums of squares of y
-    const float* ss_in;       // optional: [ss_parts][ss_ld] sums of squares of the rows, whose RMSNorm factor scales the accumulators
+    // Sums of squares, f32 of bf16 models and f64 of quantised ones (w_terms > 1), as either path is specified (src/hf/emitter_quant.rs:713-791):
+    void* ss_out;             // EPI_STORE with xp_out: [N / 128][ss_ld] of y
+    const void* ss_in;        // optional: [ss_parts][ss_ld] of the rows, whose RMSNorm factor scales the accumulators
     int ss_parts, ss_ld;
     float eps;
     // EPI_QKV_ROPE
@@ -55,7 +56,7 @@ cudaError_t launch_gemm_wide(const WideArgs& a, int sm_count, cudaStream_t st, b
 // interleave_which is 0 (gate) or 1 (up).  K a multiple of 64.
 inline int wide_quant_terms(bool q4) { return q4 ? 2 : 3; }
 cudaError_t launch_wide_pack_quant(const uint8_t* blocks, int n_rows, int K, bool q4, uint16_t* dst, int n_off, int interleave_which, cudaStream_t st);
-// f32 rows -> activation image; folds an RMSNorm (weight norm_w) when norm_w is not null.
-cudaError_t launch_wide_pack(const float* x, int ldx, int M, int K, const float* norm_w, float eps, unsigned char* xp, cudaStream_t st, bool pdl);
+// f32 rows -> activation image; folds an RMSNorm (weight norm_w, squares summed in f64 on request) when norm_w is not null.
+cudaError_t launch_wide_pack(const float* x, int ldx, int M, int K, const float* norm_w, float eps, bool f64, unsigned char* xp, cudaStream_t st, bool pdl);
 
 }  // namespace hm

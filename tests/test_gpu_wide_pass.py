@@ -94,3 +94,40 @@ def test_quantised_prompts(hm, oracle, tmp_path, gt, bias, norm, n):
     assert float(np.abs(lg - narrow).max()) <= 3e-4 * ref
     assert float(np.abs(after - m.decode_step([int(ids[n])])[0][0]).max()) <= 3e-4 * ref
     m.close()
+
+
+@pytest.mark.parametrize("dt", ["Q8_0", "Q4_0"])
+def test_norms_of_quantised_prompts_sum_in_64_bits(hm, dt):
+    # The output and down projections are zero, so every layer sees the embedding; the value projection picks elements of the normed row: the
+    # cached values are the factor's bits.  (f32 sums of the squares put about a third of the rows off by one in the last place.)
+    H, I, V, n, kvd = 256, 128, 512, 200, 128
+    cfg = hm.TransformerConfig(H, I, 4, 3, 2, V, 1e-6, 1e4, 256, True, 64)
+
+    def blocks(codes):  # [rows, K] whole numbers, scale 1
+        c = codes.reshape(-1, 32)
+        d = np.broadcast_to(np.float16(1.0).reshape(1).view(np.uint8), (len(c), 2))
+        body = c.astype(np.int8).view(np.uint8) if dt == "Q8_0" else (c[:, :16] + 8 | (c[:, 16:] + 8) << 4).astype(np.uint8)
+        return np.concatenate([d, body], 1)
+
+    rng = np.random.default_rng(3)
+    embed = synth.f32_to_bf16_rne((rng.standard_normal((V, H)) * np.exp(rng.uniform(-3, 3, (V, 1)))).astype(np.float32))
+    one = synth.f32_to_bf16_rne(np.ones(H, np.float32))
+    tensors = [("model.embed_tokens.weight", hm.DType.BF16, (V, H), embed), ("model.norm.weight", hm.DType.BF16, (H,), one)]
+    shapes = {"self_attn.q_proj": (H, H), "self_attn.k_proj": (kvd, H), "self_attn.v_proj": (kvd, H), "self_attn.o_proj": (H, H), "mlp.gate_proj": (I, H), "mlp.up_proj": (I, H), "mlp.down_proj": (H, I)}
+    for i in range(3):
+        tensors += [(f"model.layers.{i}.{k}_layernorm.weight", hm.DType.BF16, (H,), one) for k in ("input", "post_attention")]
+        for name, shape in shapes.items():
+            codes = np.zeros(shape, np.int64)
+            if "v_proj" in name:
+                codes[np.arange(kvd), 2 * np.arange(kvd)] = 1
+            tensors.append((f"model.layers.{i}.{name}.weight", hm.DType[dt], shape, blocks(codes)))
+    m = hm.HfModel.from_tensors(cfg, tensors)
+    m.init_kv_cache(256)
+    ids = synth.prompt_ids(8, n, V)
+    m.prefill(ids)
+    x = synth.bf16_to_f32(embed)[np.asarray(ids)]
+    inv = np.float32(1) / np.sqrt(((x.astype(np.float64) ** 2).sum(1) / H).astype(np.float32) + np.float32(1e-6))
+    want = (x * inv[:, None])[:, ::2].reshape(n, 2, 64).transpose(1, 0, 2)
+    for layer in range(3):
+        np.testing.assert_array_equal(m.kv_view(layer)[1][0], want)
+    m.close()
