@@ -138,6 +138,7 @@ SIGNATURES = {
     "hm_selftest_expire_wait": (_i32, [_vp]),
     "hm_engine_stream": (_vp, [_vp]),
     "hm_launches_per_step": (_i32, [_vp, _i32p]),
+    "hm_wide_rows": (_i32, [_vp, _i32p]),
     "hm_gemv_bf16": (_i32, [_vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp]),
     "hm_gemv_bf16_noalloc": (_i32, [_vp, _vp, _i32, _i32, _i32, _i32, _vp, _vp]),
     "hm_pack_bf16_slabs": (_i32, [_vp, _i32, _i32, _vp, _vp]),
@@ -420,6 +421,12 @@ class HfModel:
     def launches_per_step(self) -> int:
         v = C.c_int(0)
         _check(self._lib.hm_launches_per_step(self._h, C.byref(v)), self._h)
+        return v.value
+
+    def wide_rows(self) -> int:
+        """Rows of the last prefill or step that ran in passes of more than 64 rows."""
+        v = C.c_int(0)
+        _check(self._lib.hm_wide_rows(self._h, C.byref(v)), self._h)
         return v.value
 
     # -- KV cache --

@@ -669,6 +669,11 @@ int hm_profile_decode(hm_engine* e, int steps, hm_kernel_stat* out, int cap, int
 }
 int hm_selftest_expire_wait(hm_engine* e) { return e ? e->impl->selftest_expire_wait() : gfail(HM_ERR_INVALID, "null engine"); }
 void* hm_engine_stream(hm_engine* e) { return e ? (void*)e->impl->stream() : nullptr; }
+int hm_wide_rows(hm_engine* e, int* out) {
+    if (!e || !out) return gfail(HM_ERR_INVALID, "null argument");
+    *out = e->impl->wide_rows();
+    return HM_OK;
+}
 int hm_launches_per_step(hm_engine* e, int* out) {
     if (!e || !out) return gfail(HM_ERR_INVALID, "null argument");
     *out = e->impl->launches_per_step();

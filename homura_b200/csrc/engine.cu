@@ -1491,7 +1491,7 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
     const int chunk = (use_tc_ || quant_) ? TC_ROWS : MAX_M;
     WidePlan plan;
     if (const int wrc = plan_wide(st + n, st + 2 * n, n, &plan)) return wrc;
-    const int wide_rows = plan.rows;
+    wide_rows_ = plan.rows;
     for (const WidePass& w : plan.passes) {
         const bool last = w.row0 + w.rows >= n;
         int rc = enqueue_wide(w, pf_tokens_ + w.row0, pf_pos_ + w.row0, pf_seq_ + w.row0, &launches);
@@ -1499,7 +1499,7 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
             rc = enqueue_logits(wide_.h + (size_t)(w.rows - 1) * H_, 1, false, false, next_dev_ + seq, tokens_dev_ + seq, pos_dev_ + seq, hist_dev_ + (size_t)seq * (max_seq_ + 1), &launches);
         if (rc) return rc;
     }
-    for (int c0 = wide_rows; c0 < n; c0 += chunk) {
+    for (int c0 = plan.rows; c0 < n; c0 += chunk) {
         const int mc = std::min(chunk, n - c0);
         const bool last = c0 + mc >= n;
         pass_longest_ = len0 + c0 + mc;

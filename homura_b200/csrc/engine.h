@@ -178,6 +178,7 @@ class Engine {
     uint64_t weight_bytes() const;
     cudaStream_t stream() const { return stream_; }
     int launches_per_step() const { return launches_per_step_; }
+    int wide_rows() const { return wide_rows_; }
     std::string err;
 
    private:
@@ -356,6 +357,7 @@ class Engine {
         int32_t *tables = nullptr, *tables_host = nullptr;
         size_t table_words = 0, tiles_at = 0;
     } wide_;
+    int wide_rows_ = 0;  // rows of the last call that ran in them
 
     // listed designs
     float *mix_raw_ = nullptr, *qlat_ = nullptr, *ctx_ = nullptr;  // input projection, queries in latent space, attention result in latent space

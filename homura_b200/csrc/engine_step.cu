@@ -146,6 +146,7 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
     }
     WidePlan plan;
     if (const int wrc = plan_wide(p_pos, p_seq, (int)rows, &plan)) return wrc;
+    wide_rows_ = plan.rows;
     // passes: the wide ones, then chunks; wanted rows as indices within their pass
     struct Pass { size_t row0; int rows, wants, longest; };
     std::vector<Pass> passes;

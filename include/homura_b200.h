@@ -241,6 +241,8 @@ HM_API int hm_selftest_expire_wait(hm_engine* e);
 HM_API void* hm_engine_stream(hm_engine* e);
 /* Number of kernel launches one decode step of this engine issues. */
 HM_API int hm_launches_per_step(hm_engine* e, int* out);
+/* Rows of the last hm_prefill / hm_step (or of the prompt of hm_generate) that ran in passes of more than 64 rows. */
+HM_API int hm_wide_rows(hm_engine* e, int* out);
 
 /* ---- standalone kernels (the per-kernel sweeps) ------------------------------------- */
 /* y[M,N] = x[M,K] @ W, bf16 weights, f32 activations and accumulation: the mixed matmul of

@@ -20,10 +20,12 @@ def test_prompts_at_the_edges_of_the_tiles(hm, oracle, name, kv, n):
     ids = synth.prompt_ids(13, n + 100, cfg.vocab_size)
     want = om.forward_all(ids)
     tok, lg = m.prefill(ids[:n], want_logits=True)
+    assert m.wide_rows() == n
     assert_logits_close(lg, want[n - 1], scale_tol=exact)
     assert not exact or tok == oracle.argmax(want[n - 1])
     # the next portion starts in the middle of a page, of a block of keys, and of nothing
     got, _, _ = m.step([(0, ids[n:], np.arange(100))], want_logits=True)
+    assert m.wide_rows() == 100
     assert_logits_close(got, want[n:], scale_tol=exact)
     om.reset()
     om.prefill(ids)
@@ -47,6 +49,7 @@ def test_mixed_runs_of_any_length(hm, oracle, name, before, rows):
     want = [oracle.OracleModel.from_hf_dir(d, max_seq_len=256).forward_all(t) for t in ids]
     m.step([(i, ids[i][: before[i]], []) for i in range(n) if before[i]], want_logits=False)
     got, greedy, hidden = m.step([(i, ids[i][before[i] : before[i] + rows[i]], np.arange(rows[i])) for i in range(n)], want_logits=True, want_greedy=True, want_hidden=True)
+    assert m.wide_rows() == sum(rows)
     ref = np.concatenate([w[b : b + r] for w, b, r in zip(want, before, rows)])
     assert_logits_close(got, ref)
     assert greedy.tolist() == [oracle.argmax(r) for r in ref]
@@ -63,6 +66,7 @@ def test_prompts_of_several_passes(hm, oracle):
     m.init_kv_cache(4352)
     ids = synth.prompt_ids(3, 4200, cfg.vocab_size)
     tok, lg = m.prefill(ids, want_logits=True)
+    assert m.wide_rows() == 4200
     tok_o, lg_o = om.prefill(ids)
     assert_logits_close(lg, lg_o)
     assert tok == tok_o and m.kv_cache_len() == 4200
@@ -85,12 +89,14 @@ def test_quantised_prompts(hm, oracle, tmp_path, gt, bias, norm, n):
     ids = synth.prompt_ids(21, n + 1, cfg.vocab_size)
     _, want = om.prefill(ids[:n])
     tok, lg = m.prefill(ids[:n], want_logits=True)
+    assert m.wide_rows() == n
     ref = max(1.0, float(np.abs(want).max()))
     assert float(np.abs(lg - want).max()) <= 3e-4 * ref  # the bound of the quantised batches
     after = m.decode_step([int(ids[n])])[0][0]
     m.reset_kv_cache()
     for a in range(0, n, 60):
         _, narrow = m.prefill(ids[a : min(n, a + 60)], want_logits=True)
+        assert m.wide_rows() == 0
     assert float(np.abs(lg - narrow).max()) <= 3e-4 * ref
     assert float(np.abs(after - m.decode_step([int(ids[n])])[0][0]).max()) <= 3e-4 * ref
     m.close()
@@ -125,6 +131,7 @@ def test_norms_of_quantised_prompts_sum_in_64_bits(hm, dt):
     m.init_kv_cache(256)
     ids = synth.prompt_ids(8, n, V)
     m.prefill(ids)
+    assert m.wide_rows() == n
     x = synth.bf16_to_f32(embed)[np.asarray(ids)]
     inv = np.float32(1) / np.sqrt(((x.astype(np.float64) ** 2).sum(1) / H).astype(np.float32) + np.float32(1e-6))
     want = (x * inv[:, None])[:, ::2].reshape(n, 2, 64).transpose(1, 0, 2)
