@@ -140,7 +140,7 @@ Engine::~Engine() {
 // ---- weight loading -----------------------------------------------------------------------
 
 int Engine::stage(const void* host, size_t nbytes, void** dev) {
-    HM_CUDA(cudaMalloc(dev, nbytes));
+    HM_CUDA(dev_alloc(dev, nbytes));
     cudaError_t e = cudaMemcpyAsync(*dev, host, nbytes, cudaMemcpyHostToDevice, stream_);
     if (e != cudaSuccess) {
         cudaFree(*dev);
@@ -180,7 +180,7 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
     if (!q) {
         if (!L.slabs) {
             const size_t bytes = (size_t)((N_total + SLAB - 1) / SLAB) * K * SLAB * 2;
-            ce = cudaMalloc(&L.slabs, bytes);
+            ce = dev_alloc(&L.slabs, bytes);
             if (ce == cudaSuccess) ce = cudaMemsetAsync(L.slabs, 0, bytes, stream_);
         }
         if (ce == cudaSuccess) ce = launch_pack_slabs_from_nk((const uint16_t*)tmp, n_part, K, L.slabs, n_off, interleave_which, stream_);
@@ -188,7 +188,7 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
             // second copy for passes over more than four rows (same 64 + 64 gate/up interleave per 128 features)
             if (!L.tc) {
                 const size_t bytes = tc_packed_elems(K, N_total) * 2;
-                ce = cudaMalloc(&L.tc, bytes);
+                ce = dev_alloc(&L.tc, bytes);
                 if (ce == cudaSuccess) ce = cudaMemsetAsync(L.tc, 0, bytes, stream_);
             }
             if (ce == cudaSuccess) ce = launch_pack_tc((const uint16_t*)tmp, n_part, K, false, L.tc, n_off, interleave_which, stream_);
@@ -208,8 +208,8 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
     if (!q) {
     } else if (kq) {
         if (!L.kq_data) {
-            ce = cudaMalloc(&L.kq_data, kquant_data_bytes(K, N_total));
-            if (ce == cudaSuccess) ce = cudaMalloc(&L.kq_tile_type, kquant_tiles(N_total));
+            ce = dev_alloc(&L.kq_data, kquant_data_bytes(K, N_total));
+            if (ce == cudaSuccess) ce = dev_alloc(&L.kq_tile_type, kquant_tiles(N_total));
             if (ce == cudaSuccess) ce = cudaMemsetAsync(L.kq_data, 0, kquant_data_bytes(K, N_total), stream_);
             if (ce == cudaSuccess) ce = cudaMemsetAsync(L.kq_tile_type, 0, kquant_tiles(N_total), stream_);
         }
@@ -226,16 +226,16 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
     } else {
         const int q4 = dtype == HM_Q4_0;
         if (!L.scales) {
-            ce = cudaMalloc(&L.scales, quant_scale_elems(K, N_total) * 2);
-            if (ce == cudaSuccess) ce = cudaMalloc(&L.codes, quant_code_bytes(K, N_total, q4));
+            ce = dev_alloc(&L.scales, quant_scale_elems(K, N_total) * 2);
+            if (ce == cudaSuccess) ce = dev_alloc(&L.codes, quant_code_bytes(K, N_total, q4));
             if (ce == cudaSuccess) ce = cudaMemsetAsync(L.scales, 0, quant_scale_elems(K, N_total) * 2, stream_);
             if (ce == cudaSuccess) ce = cudaMemsetAsync(L.codes, 0, quant_code_bytes(K, N_total, q4), stream_);
         }
         if (ce == cudaSuccess) ce = launch_split_blocks((const uint8_t*)tmp, n_part, K, q4, n_off, interleave_which, L.scales, L.codes, stream_, rope_hd);
         quant_ = true;
-        // a second copy for prompts (4 or 6 bytes per weight); without the memory for it prompts run in passes of 64 rows
-        if (ce == cudaSuccess && use_tc_ && &L != &lm_head_ && K % 64 == 0 && wide_copies_fit(wide_quant_terms(q4))) {
-            if (!L.wide && L.loaded_parts == 0) {
+        // a second copy for prompts (4 or 6 bytes per weight); without the memory for all of them prompts run in passes of 64 rows
+        if (ce == cudaSuccess && &L != &lm_head_ && wide_copies(wide_quant_terms(q4))) {
+            if (!L.wide) {
                 L.wide_terms = wide_quant_terms(q4);
                 const size_t bytes = tc_packed_elems(K, N_total) * 2 * L.wide_terms;
                 if (cudaMalloc(&L.wide, bytes) == cudaSuccess) {
@@ -243,6 +243,7 @@ int Engine::load_linear(LinearW& L, int K, int N_total, int n_off, int n_part, i
                 } else {
                     cudaGetLastError();
                     L.wide = nullptr;
+                    give_back();
                 }
             }
             if (ce == cudaSuccess && L.wide) ce = launch_wide_pack_quant((const uint8_t*)tmp, n_part, K, q4, L.wide, n_off, interleave_which, stream_);
@@ -260,7 +261,7 @@ int Engine::load_vec_f32(float** dst, size_t n_total, size_t off, int dtype, con
     if (!esz) return fail(HM_ERR_UNSUPPORTED, "norm / bias tensors must be f32, bf16 or f16");
     if (nbytes != n * esz || off + n > n_total) return fail(HM_ERR_INVALID, "tensor byte size does not match its shape");
     if (!*dst) {
-        HM_CUDA(cudaMalloc(dst, n_total * 4));
+        HM_CUDA(dev_alloc(dst, n_total * 4));
         HM_CUDA(cudaMemsetAsync(*dst, 0, n_total * 4, stream_));
     }
     void* tmp = nullptr;
@@ -322,7 +323,7 @@ int Engine::load_tensor(const char* cname, int dtype, const int64_t* shape, int 
             void* tmp = nullptr;
             int rc = stage(host, nbytes, &tmp);
             if (rc) return rc;
-            cudaError_t ce = cudaMalloc(&embed_, n * 4);
+            cudaError_t ce = dev_alloc(&embed_, n * 4);
             if (ce == cudaSuccess) ce = launch_dequant((const uint8_t*)tmp, n / 32, dtype == HM_Q4_0, (float*)embed_, stream_);
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream_);
             cudaFree(tmp);
@@ -333,7 +334,7 @@ int Engine::load_tensor(const char* cname, int dtype, const int64_t* shape, int 
             void* tmp = nullptr;
             int rc = stage(host, nbytes, &tmp);
             if (rc) return rc;
-            cudaError_t ce = cudaMalloc(&embed_, n * 4);
+            cudaError_t ce = dev_alloc(&embed_, n * 4);
             if (ce == cudaSuccess) ce = launch_dequant_k((const uint8_t*)tmp, n / 256, dtype == HM_Q6_K, (float*)embed_, stream_);
             if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream_);
             cudaFree(tmp);
@@ -418,8 +419,8 @@ int Engine::finalize() {
     if (!spec_.listed()) {
         std::vector<float> c, s;
         build_rope_table(hd_, cfg_.max_position_embeddings, cfg_.rope_theta, &c, &s);
-        HM_CUDA(cudaMalloc(&rope_cos_, c.size() * 4));
-        HM_CUDA(cudaMalloc(&rope_sin_, s.size() * 4));
+        HM_CUDA(dev_alloc(&rope_cos_, c.size() * 4));
+        HM_CUDA(dev_alloc(&rope_sin_, s.size() * 4));
         HM_CUDA(cudaMemcpy(rope_cos_, c.data(), c.size() * 4, cudaMemcpyHostToDevice));
         HM_CUDA(cudaMemcpy(rope_sin_, s.data(), s.size() * 4, cudaMemcpyHostToDevice));
     }
@@ -427,12 +428,12 @@ int Engine::finalize() {
         // pair i of the position vector turns by 10000^(-2 i / width) radians per position
         std::vector<double> t((H_ + 1) / 2);
         for (size_t i = 0; i < t.size(); ++i) t[i] = std::pow(10000.0, -2.0 * (double)i / H_) / 6.283185307179586;
-        HM_CUDA(cudaMalloc(&turns_, t.size() * 8));
+        HM_CUDA(dev_alloc(&turns_, t.size() * 8));
         HM_CUDA(cudaMemcpy(turns_, t.data(), t.size() * 8, cudaMemcpyHostToDevice));
     }
-    HM_CUDA(cudaMalloc(&err_flag_, 4));
+    HM_CUDA(dev_alloc(&err_flag_, 4));
     HM_CUDA(cudaMemset(err_flag_, 0, 4));
-    HM_CUDA(cudaMalloc(&fin_ticket_, 4));
+    HM_CUDA(dev_alloc(&fin_ticket_, 4));
     HM_CUDA(cudaMemset(fin_ticket_, 0, 4));
     finalized_ = true;
     return HM_OK;
@@ -454,7 +455,7 @@ int Engine::ensure_scratch(int rows) {
     auto re = [&](auto** p, size_t count) -> cudaError_t {
         if (*p) cudaFree(*p);
         *p = nullptr;
-        cudaError_t e = cudaMalloc((void**)p, count * sizeof(**p));
+        cudaError_t e = dev_alloc((void**)p, count * sizeof(**p));
         if (e == cudaSuccess) e = cudaMemset(*p, 0, count * sizeof(**p));
         return e;
     };
@@ -547,8 +548,8 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
         if (rc) return rc;
     }
     for (int l = 0; l < L_ && !spec_.listed(); ++l) {
-        HM_CUDA(cudaMalloc(&k_pool_[l], pool_bytes));
-        HM_CUDA(cudaMalloc(&v_pool_[l], pool_bytes));
+        HM_CUDA(dev_alloc(&k_pool_[l], pool_bytes));
+        HM_CUDA(dev_alloc(&v_pool_[l], pool_bytes));
         HM_CUDA(cudaMemset(k_pool_[l], 0, pool_bytes));
         HM_CUDA(cudaMemset(v_pool_[l], 0, pool_bytes));
     }
@@ -561,7 +562,7 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
         st ^= st << 13; st ^= st >> 7; st ^= st << 17;
         std::swap(perm[i - 1], perm[st % i]);
     }
-    HM_CUDA(cudaMalloc(&page_table_, table_len * 4));
+    HM_CUDA(dev_alloc(&page_table_, table_len * 4));
     pooled_ = pool_tokens > 0;
     free_pages_.clear();
     seq_pages_.assign(batch, {});
@@ -573,27 +574,27 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     }
     std::vector<int32_t> iota(std::max(batch, TC_ROWS));
     for (size_t i = 0; i < iota.size(); ++i) iota[i] = (int32_t)i;
-    HM_CUDA(cudaMalloc(&seq_iota_, iota.size() * 4));
+    HM_CUDA(dev_alloc(&seq_iota_, iota.size() * 4));
     HM_CUDA(cudaMemcpy(seq_iota_, iota.data(), iota.size() * 4, cudaMemcpyHostToDevice));
-    HM_CUDA(cudaMalloc(&pos_dev_, batch * 4));
+    HM_CUDA(dev_alloc(&pos_dev_, batch * 4));
     HM_CUDA(cudaMemset(pos_dev_, 0, batch * 4));
-    HM_CUDA(cudaMalloc(&tokens_dev_, batch * 4));
+    HM_CUDA(dev_alloc(&tokens_dev_, batch * 4));
     HM_CUDA(cudaMemset(tokens_dev_, 0, batch * 4));
-    HM_CUDA(cudaMalloc(&next_dev_, batch * 4));
+    HM_CUDA(dev_alloc(&next_dev_, batch * 4));
     HM_CUDA(cudaMemset(next_dev_, 0, batch * 4));
-    HM_CUDA(cudaMalloc(&hist_dev_, (size_t)batch * (max_seq_len + 1) * 4));
+    HM_CUDA(dev_alloc(&hist_dev_, (size_t)batch * (max_seq_len + 1) * 4));
     HM_CUDA(cudaMemset(hist_dev_, 0, (size_t)batch * (max_seq_len + 1) * 4));
-    HM_CUDA(cudaMalloc(&pf_tokens_, (size_t)max_seq_len * 4));
-    HM_CUDA(cudaMalloc(&pf_pos_, (size_t)max_seq_len * 4));
-    HM_CUDA(cudaMalloc(&pf_seq_, (size_t)max_seq_len * 4));
+    HM_CUDA(dev_alloc(&pf_tokens_, (size_t)max_seq_len * 4));
+    HM_CUDA(dev_alloc(&pf_pos_, (size_t)max_seq_len * 4));
+    HM_CUDA(dev_alloc(&pf_seq_, (size_t)max_seq_len * 4));
     pin_u32_cap_ = std::max<size_t>((size_t)3 * max_seq_len, (size_t)batch * (max_seq_len + 6)) + 16;  // the last word receives the device error word
     HM_CUDA(cudaMallocHost(&pin_u32_, pin_u32_cap_ * 4));
     pin_u32_[pin_u32_cap_ - 1] = 0;
-    HM_CUDA(cudaMalloc(&smp_rng_, (size_t)batch * 8));
+    HM_CUDA(dev_alloc(&smp_rng_, (size_t)batch * 8));
     HM_CUDA(cudaMemset(smp_rng_, 0, (size_t)batch * 8));
-    HM_CUDA(cudaMalloc(&smp_gen_start_, (size_t)batch * 4));
+    HM_CUDA(dev_alloc(&smp_gen_start_, (size_t)batch * 4));
     HM_CUDA(cudaMemset(smp_gen_start_, 0, (size_t)batch * 4));
-    HM_CUDA(cudaMalloc(&smp_overflow_, (size_t)batch * 4));
+    HM_CUDA(dev_alloc(&smp_overflow_, (size_t)batch * 4));
     HM_CUDA(cudaMemset(smp_overflow_, 0, (size_t)batch * 4));
     len_.assign(batch, 0);
     gen_start_.assign(batch, 0);
@@ -613,15 +614,15 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     att_cluster_ = use_clusters_ && max_pages_ <= 64 && (long)batch * kvh_ < sm_count_ / 2;
     att_nsplit_ = att_cluster_ ? attn_pick_cluster(max_pages_, std::min(max_cluster_, 16)) : attn_pick_nsplit(batch, kvh_, max_pages_, sm_count_, kv_bf16_);
     if (!spec_.listed()) {
-        HM_CUDA(cudaMalloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * hd_ * 4));
-        HM_CUDA(cudaMalloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * 2 * 4));
-        HM_CUDA(cudaMalloc(&att_tickets_, (size_t)scratch_rows_ * kvh_ * 4));
+        HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * hd_ * 4));
+        HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * 2 * 4));
+        HM_CUDA(dev_alloc(&att_tickets_, (size_t)scratch_rows_ * kvh_ * 4));
         HM_CUDA(cudaMemset(att_tickets_, 0, (size_t)scratch_rows_ * kvh_ * 4));
     }
 #ifdef HM_PHASE_TRACE
     if (const char* gt = std::getenv("HM_GEMV_TRACE")) {
         if (gt[0] == '1' && !gemv_trace_) {
-            HM_CUDA(cudaMalloc(&gemv_trace_, 512 * 16 * sizeof(unsigned long long)));
+            HM_CUDA(dev_alloc(&gemv_trace_, 512 * 16 * sizeof(unsigned long long)));
             HM_CUDA(cudaMemset(gemv_trace_, 0, 512 * 16 * sizeof(unsigned long long)));
         }
     }
@@ -716,11 +717,11 @@ int Engine::kv_append(int seq, int layer, const float* k_rows, const float* v_ro
         const size_t bytes = (size_t)kvh_ * n_new * hd_ * 4;
         float *dk = nullptr, *dv = nullptr;
         if (k_rows) {
-            HM_CUDA(cudaMalloc(&dk, bytes));
+            HM_CUDA(dev_alloc(&dk, bytes));
             HM_CUDA(cudaMemcpyAsync(dk, k_rows, bytes, cudaMemcpyHostToDevice, stream_));
         }
         if (v_rows) {
-            HM_CUDA(cudaMalloc(&dv, bytes));
+            HM_CUDA(dev_alloc(&dv, bytes));
             HM_CUDA(cudaMemcpyAsync(dv, v_rows, bytes, cudaMemcpyHostToDevice, stream_));
         }
         KvDesc kv{k_pool_[layer], v_pool_[layer], page_table_, max_pages_, page_tokens_, kvh_, hd_, kv_bf16_ ? 1 : 0};
@@ -748,8 +749,8 @@ int Engine::kv_view(int seq, int layer, float* k_out, float* v_out) {
     if (len == 0) return HM_OK;
     const size_t k_bytes = (size_t)(ls ? ls->kv_heads * ls->dim : kvh_ * hd_) * len * 4, v_bytes = (size_t)(ls ? ls->kv_heads * ls->vdim : kvh_ * hd_) * len * 4;
     float *dk = nullptr, *dv = nullptr;
-    HM_CUDA(cudaMalloc(&dk, k_bytes));
-    HM_CUDA(cudaMalloc(&dv, v_bytes));
+    HM_CUDA(dev_alloc(&dk, k_bytes));
+    HM_CUDA(dev_alloc(&dv, v_bytes));
     KvDesc kv{k_pool_[layer], v_pool_[layer], page_table_, max_pages_, page_tokens_, kvh_, hd_, kv_bf16_ ? 1 : 0};
     cudaError_t ce = ls ? launch_gqa_read(gqa_pool(layer), seq, len, dk, dv, stream_) : launch_kv_read_rows(kv, seq, len, dk, dv, stream_);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(k_out, dk, k_bytes, cudaMemcpyDeviceToHost, stream_);
@@ -1823,8 +1824,8 @@ uint32_t host_sample_token(const float* logits, int n, const hm_sampling& cfg, c
 
 int Engine::ensure_sampler_scratch() {
     if (smp_scaled_) return HM_OK;
-    HM_CUDA(cudaMalloc(&smp_scaled_, (size_t)batch_ * V_ * 4));
-    HM_CUDA(cudaMalloc(&smp_count_, (size_t)batch_ * V_ * 4));
+    HM_CUDA(dev_alloc(&smp_scaled_, (size_t)batch_ * V_ * 4));
+    HM_CUDA(dev_alloc(&smp_count_, (size_t)batch_ * V_ * 4));
     HM_CUDA(cudaMemset(smp_count_, 0, (size_t)batch_ * V_ * 4));
     return HM_OK;
 }

@@ -196,9 +196,21 @@ class Engine {
     int enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_pos, const int32_t* row_seq, int lm_row0, int lm_rows, bool advance, uint32_t* next_dev, uint32_t* feed_dev, int32_t* pos_dev, uint32_t* hist_dev, int* launches);
     int enqueue_logits(const float* x, int lm_rows, bool whole_pass, bool packed, uint32_t* next_dev, uint32_t* feed_dev, int32_t* pos_dev, uint32_t* hist_dev, int* launches);
     AttnArgs attn_args(int l, int M, const float* q, const int32_t* row_pos, const int32_t* row_seq) const;
+    // Memory that a call cannot do without: what the engine holds for speed alone is given back for it.
+    template <typename T>
+    cudaError_t dev_alloc(T** p, size_t bytes) {
+        cudaError_t e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            if (give_back()) e = cudaMalloc(p, bytes);
+        }
+        return e;
+    }
     // passes over many rows (engine_wide.cu)
     bool wide_fits() const;
-    bool wide_copies_fit(int terms) const;
+    bool wide_sizes() const;
+    bool wide_copies(int terms);
+    bool give_back();
     bool ensure_wide(int rows);
     int plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan);
     int enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches);
@@ -357,6 +369,7 @@ class Engine {
         int32_t *tables = nullptr, *tables_host = nullptr;
         size_t table_words = 0, tiles_at = 0;
     } wide_;
+    int wide_copies_ = -1;  // copies of quantised weights for them: not decided yet, none, all
     int wide_rows_ = 0;  // rows of the last call that ran in them
 
     // listed designs

@@ -119,7 +119,7 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
         auto re = [&](auto** p) -> cudaError_t {
             if (*p) cudaFree(*p);
             *p = nullptr;
-            return cudaMalloc((void**)p, cap * 4);
+            return dev_alloc((void**)p, cap * 4);
         };
         st_rows_ = 0;
         HM_CUDA(re(&st_tokens_));

@@ -18,24 +18,43 @@ constexpr int WIDE_MIN_RUN = 8;
 // Staged keys and values of one launch at most (one sequence may take more).
 constexpr size_t WIDE_STAGED = 512u << 20;
 
+// Sizes that the wide passes take.
+bool Engine::wide_sizes() const { return !spec_.listed() && use_tc_ && H_ % 128 == 0 && I_ % 64 == 0; }
+
 bool Engine::wide_fits() const {
-    if (spec_.listed() || !use_tc_ || H_ % 128 != 0 || I_ % 64 != 0 || page_tokens_ != 16) return false;
+    if (!wide_sizes() || page_tokens_ != 16) return false;
     for (const LayerW& l : layers_)
         for (const LinearW* w : {&l.qkv, &l.o, &l.gu, &l.down})
             if (!w->tc && !w->wide) return false;
     return true;
 }
 
-// Whether all projections of a quantised model may be held as bf16 terms as well: in at most an eighth of the GPU's memory (22 GB: models
-// of up to 3.8 B weights in Q8_0), so that models near its limits keep it for their caches.
-bool Engine::wide_copies_fit(int terms) const {
-    size_t free_bytes = 0, total = 0;
-    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+// Whether the projections of a quantised model are held as bf16 terms as well.  Decided once, when the first of them is loaded, so that a model
+// has all copies or none: where the wide passes take its sizes, and the copies take an eighth of the free memory at most (of a GPU of its
+// own 22 GB: models of up to 3.8 B weights in Q8_0).  The rest of the weights, a fifth of the copies at most, and the caches find room beside them.
+bool Engine::wide_copies(int terms) {
+    if (wide_copies_ < 0) {
+        size_t free_bytes = 0, total = 0;
+        const double weights = (double)L_ * ((double)H_ * (2.0 * qdim_ + 2.0 * kvdim_) + 3.0 * H_ * I_);
+        const bool known = cudaMemGetInfo(&free_bytes, &total) == cudaSuccess;
+        if (!known) cudaGetLastError();
+        wide_copies_ = known && wide_sizes() && weights * 2 * terms <= (double)free_bytes / 8;
     }
-    const double weights = (double)L_ * ((double)H_ * (2.0 * qdim_ + 2.0 * kvdim_) + 3.0 * H_ * I_);
-    return weights * 2 * terms <= (double)total / 8;
+    return wide_copies_ > 0;
+}
+
+// Frees what the engine can do without: the wide passes' scratch and a quantised model's copies (its prompts then run in passes of 64 rows).
+// The calls that allocate do so before they plan a pass.  False: there was nothing.
+bool Engine::give_back() {
+    bool any = wide_.cap > 0 || wide_copies_ > 0;
+    if (stream_) cudaStreamSynchronize(stream_);
+    free_wide();
+    each_linear([&](LinearW& w) {
+        if (w.wide) cudaFree(w.wide);
+        w.wide = nullptr;
+    });
+    if (wide_copies_ > 0) wide_copies_ = 0;
+    return any;
 }
 
 void Engine::free_wide() {
