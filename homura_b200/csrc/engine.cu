@@ -588,7 +588,7 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     HM_CUDA(dev_alloc(&pf_pos_, (size_t)max_seq_len * 4));
     HM_CUDA(dev_alloc(&pf_seq_, (size_t)max_seq_len * 4));
     pin_u32_cap_ = std::max<size_t>((size_t)3 * max_seq_len, (size_t)batch * (max_seq_len + 6)) + 16;  // the last word receives the device error word
-    HM_CUDA(cudaMallocHost(&pin_u32_, pin_u32_cap_ * 4));
+    HM_CUDA(cudaMallocHost(&pin_u32_, (pin_u32_cap_ + WIDE_TABLE) * 4));
     pin_u32_[pin_u32_cap_ - 1] = 0;
     HM_CUDA(dev_alloc(&smp_rng_, (size_t)batch * 8));
     HM_CUDA(cudaMemset(smp_rng_, 0, (size_t)batch * 8));
@@ -627,6 +627,7 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
         }
     }
 #endif
+    ensure_wide();
     return capture_decode_graph();
 }
 
@@ -647,7 +648,6 @@ int Engine::kv_free() {
     };
     for (void*& p : k_pool_) fr(p);
     for (void*& p : v_pool_) fr(p);
-    free_wide();
     k_pool_.clear();
     v_pool_.clear();
     free_listed_cache();
@@ -1495,7 +1495,7 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
     wide_rows_ = plan.rows;
     for (const WidePass& w : plan.passes) {
         const bool last = w.row0 + w.rows >= n;
-        int rc = enqueue_wide(w, pf_tokens_ + w.row0, pf_pos_ + w.row0, pf_seq_ + w.row0, &launches);
+        int rc = enqueue_wide(plan, w, pf_tokens_ + w.row0, pf_pos_ + w.row0, pf_seq_ + w.row0, &launches);
         if (rc == HM_OK && last)
             rc = enqueue_logits(wide_.h + (size_t)(w.rows - 1) * H_, 1, false, false, next_dev_ + seq, tokens_dev_ + seq, pos_dev_ + seq, hist_dev_ + (size_t)seq * (max_seq_ + 1), &launches);
         if (rc) return rc;

@@ -138,6 +138,10 @@ struct WidePass {
 struct WidePlan {
     std::vector<WidePass> passes;
     int rows = 0;  // rows that they cover; what is left at the end of the call is few
+    // on the device: the tables of all passes' attention, and room for a launch's staged keys and values
+    PrefillTile* tiles = nullptr;
+    PrefillBlock* blocks = nullptr;
+    unsigned char* staged = nullptr;
 };
 
 class Engine {
@@ -211,9 +215,9 @@ class Engine {
     bool wide_sizes() const;
     bool wide_copies(int terms);
     bool give_back();
-    bool ensure_wide(int rows);
+    bool ensure_wide();
     int plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan);
-    int enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches);
+    int enqueue_wide(const WidePlan& plan, const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches);
     void free_wide();
     int enqueue_linear(const LinearW& L, int M, const float* x, int ldx, int pro, const float* norm_w, int epi, float* y, int ldy, const float* bias, const float* resid, int layer, const int32_t* row_pos, const int32_t* row_seq, float* amax_val, int32_t* amax_idx, int* launches, const struct ArgmaxFold* fold = nullptr, const LinOpt* opt = nullptr);
     // listed designs (engine_listed.cu)
@@ -357,17 +361,20 @@ class Engine {
     int* err_flag_ = nullptr;
     unsigned int* fin_ticket_ = nullptr;  // ticket of the LM head's folded argmax
 
-    // passes over many rows: activations, activation images (gemm_wide.h), partial tiles, staged keys and values, tables
+    // Passes over many rows: activations, activation images (gemm_wide.h), partial tiles, staged keys and values, tables, all parts of one
+    // allocation; and what a call took beside it.
+    static constexpr size_t WIDE_TABLE = 4096;  // words of the kept table, also behind the pinned words of pin_u32_
     struct Wide {
-        int cap = 0;                     // rows
+        int cap = 0;  // rows
+        unsigned char* base = nullptr;
         float *h = nullptr, *q = nullptr;
         double *ss = nullptr, *ss2 = nullptr;
         unsigned char *x = nullptr, *x2 = nullptr, *att = nullptr, *act = nullptr;
         float* part = nullptr;
-        unsigned char* staged = nullptr;
-        size_t staged_bytes = 0;
-        int32_t *tables = nullptr, *tables_host = nullptr;
-        size_t table_words = 0, tiles_at = 0;
+        unsigned char *kept_staged = nullptr, *own_staged = nullptr;
+        size_t kept_bytes = 0, own_bytes = 0;
+        int32_t *kept_tables = nullptr, *own_tables = nullptr;
+        size_t own_words = 0;
     } wide_;
     int wide_copies_ = -1;  // copies of quantised weights for them: not decided yet, none, all
     int wide_rows_ = 0;  // rows of the last call that ran in them

@@ -187,7 +187,7 @@ int Engine::step(const hm_step_entry* entries, int n, float* logits, uint32_t* g
         const int mc = passes[i].rows, nw = logits || greedy ? passes[i].wants : 0;
         tap_row0_ = c0;
         if (i < plan.passes.size()) {
-            rc = enqueue_wide(plan.passes[i], st_tokens_ + c0, st_pos_ + c0, st_seq_ + c0, &launches);
+            rc = enqueue_wide(plan, plan.passes[i], st_tokens_ + c0, st_pos_ + c0, st_seq_ + c0, &launches);
             for (int w = 0; w < nw && rc == HM_OK; w += chunk) {
                 const int g = std::min(chunk, nw - w);
                 const cudaError_t ce = launch_gather_rows(wide_.h, st_want_ + done, g, H_, hsel_, stream_, pdl_);

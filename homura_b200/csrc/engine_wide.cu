@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "engine.h"
@@ -15,8 +16,8 @@ namespace hm {
 // Runs shorter than this go to the decode attention, row by row: a tile of the prompt attention costs as much for one row as for 64,
 // and its context is staged first.
 constexpr int WIDE_MIN_RUN = 8;
-// Staged keys and values of one launch at most (one sequence may take more).
-constexpr size_t WIDE_STAGED = 512u << 20;
+// Staged keys and values of one launch at most (one sequence may take more), and what is kept for them; a call that stages more takes its own.
+constexpr size_t WIDE_STAGED = 512u << 20, WIDE_STAGED_KEPT = 64u << 20;
 
 // Sizes that the wide passes take.
 bool Engine::wide_sizes() const { return !spec_.listed() && use_tc_ && H_ % 128 == 0 && I_ % 64 == 0; }
@@ -58,45 +59,68 @@ bool Engine::give_back() {
 }
 
 void Engine::free_wide() {
-    for (void* p : {(void*)wide_.h, (void*)wide_.q, (void*)wide_.ss, (void*)wide_.ss2, (void*)wide_.x, (void*)wide_.x2, (void*)wide_.att, (void*)wide_.act, (void*)wide_.part, (void*)wide_.staged, (void*)wide_.tables})
+    for (void* p : {(void*)wide_.base, (void*)wide_.own_staged, (void*)wide_.own_tables})
         if (p) cudaFree(p);
-    if (wide_.tables_host) cudaFreeHost(wide_.tables_host);
     wide_ = Wide();
 }
 
-// Scratch of a pass over `rows` rows (the stream is idle).  False without memory for it: the caller then takes passes of 64 rows.
-bool Engine::ensure_wide(int rows) {
-    if (rows <= wide_.cap) return true;
-    const int cap = std::min(WIDE_ROWS, (rows + 511) / 512 * 512), blocks = wide_blocks(cap);
-    size_t part = 1;
+// Scratch of the passes that a call on this cache can ask for, in one allocation (the stream is idle).  Taken with the cache and kept for the
+// next one: an allocation takes 0.35 ms whatever its size, and eleven of them, with pinned memory for the tables, in a prompt's first
+// pass took longer than the pass saves up to 200 tokens (the first 100 tokens of a cache, 0.5 B stack: 2.33 ms in passes of 64 rows, 2.06 here, 4.9 with them).
+// False without memory for it: the caller then takes passes of 64 rows.
+bool Engine::ensure_wide() {
+    const long all = (long)batch_ * max_seq_;
+    if (all <= TC_ROWS || !wide_fits()) return false;
+    const int rows = (int)std::min<long>(WIDE_ROWS, (all + WIDE_BLOCK - 1) / WIDE_BLOCK * WIDE_BLOCK), blocks = wide_blocks(rows);
+    const size_t staged = std::min(WIDE_STAGED_KEPT, (size_t)batch_ * ((max_seq_ + PREFILL_TILE - 1) / PREFILL_TILE) * prefill_block_bytes(kvh_, hd_, kv_bf16_));
+    if (rows <= wide_.cap && staged <= wide_.kept_bytes) return true;
+    free_wide();
+    size_t part = 1, bytes = 0;
     for (int b = 1; b <= blocks; ++b)
         for (const LinearW* w : {&layers_[0].qkv, &layers_[0].o, &layers_[0].gu, &layers_[0].down})
             part = std::max(part, wide_split(b * WIDE_BLOCK, w->K, w->N, w->tc ? 1 : w->wide_terms, w == &layers_[0].gu ? EPI_SWIGLU : EPI_STORE, sm_count_).part_floats);
-    free_wide();
-    auto get = [&](auto** p, size_t count) { return cudaMalloc((void**)p, count * sizeof(**p)) == cudaSuccess; };
-    const bool ok = get(&wide_.h, (size_t)cap * H_) && get(&wide_.q, (size_t)cap * qdim_) && get(&wide_.ss, (size_t)(H_ / 128) * cap) && get(&wide_.ss2, (size_t)(H_ / 128) * cap) &&
-                    get(&wide_.x, blocks * wide_block_bytes(H_)) && get(&wide_.x2, blocks * wide_block_bytes(H_)) && get(&wide_.att, blocks * wide_block_bytes(qdim_)) && get(&wide_.act, blocks * wide_block_bytes(I_)) &&
-                    get(&wide_.part, part);
-    if (!ok) {
+    auto place = [&](auto** p, size_t count) {  // without a base: sizes only
+        *p = wide_.base ? reinterpret_cast<std::remove_reference_t<decltype(*p)>>(wide_.base + bytes) : nullptr;
+        bytes += (count * sizeof(**p) + 1023) / 1024 * 1024;
+    };
+    auto lay = [&]() {
+        bytes = 0;
+        place(&wide_.h, (size_t)rows * H_);
+        place(&wide_.q, (size_t)rows * qdim_);
+        place(&wide_.ss, (size_t)(H_ / 128) * rows);
+        place(&wide_.ss2, (size_t)(H_ / 128) * rows);
+        place(&wide_.x, blocks * wide_block_bytes(H_));
+        place(&wide_.x2, blocks * wide_block_bytes(H_));
+        place(&wide_.att, blocks * wide_block_bytes(qdim_));
+        place(&wide_.act, blocks * wide_block_bytes(I_));
+        place(&wide_.part, part);
+        place(&wide_.kept_staged, staged);
+        place(&wide_.kept_tables, WIDE_TABLE);
+    };
+    lay();
+    if (cudaMalloc((void**)&wide_.base, bytes) != cudaSuccess) {
         cudaGetLastError();
-        free_wide();
+        wide_ = Wide();
         return false;
     }
-    wide_.cap = cap;
+    lay();
+    wide_.cap = rows;
+    wide_.kept_bytes = staged;
     return true;
 }
 
-// Rows from which a call takes wide passes: more than one 64-row pass.  Prompts of 96 rows (two passes of the 64-row kernels): 0.5 B
-// 2.44 -> 1.83 ms, 1.5 B 4.28 -> 3.08; of 128: 2.63 -> 2.00, 4.64 -> 3.23; of 65 on TinyLlama Q8_0 4.23 -> 2.87, Q4_0 4.64 -> 2.52.
+// Rows from which a call takes wide passes: more than one 64-row pass.  One prompt, ms in passes of the 64-row kernels and here: of 100 rows
+// 0.5 B 2.30 and 2.00, 1.5 B 3.51 and 3.27, TinyLlama Q8_0 6.77 and 2.95; of 65 rows 1.86 and 1.87, 3.0 to 3.8 (by the cache's capacity) and 3.07 to
+// 3.20, 4.03 and 2.94.  Single tokens of as many sequences, row by row in the attention: 65 of 1.5 B 6.5 and 3.5, of 0.5 B 3.0 and 2.3, of TinyLlama Q8_0 4.6 and
+// 3.3; 64 of them and a prompt of 20: 4.15 and 4.24, 2.88 and 2.74, 7.3 and 3.8.
 // Cuts the n rows of a call (host arrays: position and sequence of each; a sequence's rows are consecutive) into wide passes and sends
 // the tables of their attention to the device.  No passes where the rows are few or the model has no wide path.
 int Engine::plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan* plan) {
     plan->passes.clear();
     plan->rows = 0;
-    if (n <= TC_ROWS || !wide_fits()) return HM_OK;
+    if (n <= TC_ROWS || !ensure_wide()) return HM_OK;
     const int n_pass = (n + WIDE_ROWS - 1) / WIDE_ROWS;
     const int per = std::min(WIDE_ROWS, ((n + n_pass - 1) / n_pass + WIDE_BLOCK - 1) / WIDE_BLOCK * WIDE_BLOCK);
-    if (!ensure_wide(std::min(per, n))) return HM_OK;
     const size_t block_bytes = prefill_block_bytes(kvh_, hd_, kv_bf16_);
     const int budget = (int)std::max<size_t>(1, WIDE_STAGED / block_bytes);
     std::vector<PrefillTile> tiles;
@@ -144,34 +168,43 @@ int Engine::plan_wide(const uint32_t* pos, const uint32_t* seq, int n, WidePlan*
         plan->rows = 0;
         return HM_OK;
     };
-    if (words > wide_.table_words) {
-        if (wide_.tables) cudaFree(wide_.tables);
-        if (wide_.tables_host) cudaFreeHost(wide_.tables_host);
-        wide_.tables = wide_.tables_host = nullptr;
-        wide_.table_words = 0;
-        const size_t cap = std::max<size_t>(4096, words + words / 2);
-        if (cudaMalloc((void**)&wide_.tables, cap * 4) != cudaSuccess || cudaMallocHost((void**)&wide_.tables_host, cap * 4) != cudaSuccess) return give_up();
-        wide_.table_words = cap;
+    // what the kept parts do not hold (passes of many thousand tokens) is allocated once and grows
+    if (words > WIDE_TABLE && words > wide_.own_words) {
+        if (wide_.own_tables) cudaFree(wide_.own_tables);
+        wide_.own_tables = nullptr;
+        wide_.own_words = 0;
+        const size_t cap = words + words / 2;
+        if (cudaMalloc((void**)&wide_.own_tables, cap * 4) != cudaSuccess) return give_up();
+        wide_.own_words = cap;
     }
-    if (most * block_bytes > wide_.staged_bytes) {
-        if (wide_.staged) cudaFree(wide_.staged);
-        wide_.staged = nullptr;
-        wide_.staged_bytes = 0;
+    if (most * block_bytes > std::max(wide_.kept_bytes, wide_.own_bytes)) {
+        if (wide_.own_staged) cudaFree(wide_.own_staged);
+        wide_.own_staged = nullptr;
+        wide_.own_bytes = 0;
         const size_t bytes = std::max<size_t>(most * block_bytes, std::min<size_t>(WIDE_STAGED, 2 * most * block_bytes));
-        if (cudaMalloc((void**)&wide_.staged, bytes) != cudaSuccess) return give_up();
-        wide_.staged_bytes = bytes;
+        if (cudaMalloc((void**)&wide_.own_staged, bytes) != cudaSuccess) return give_up();
+        wide_.own_bytes = bytes;
     }
-    if (words) {
-        std::memcpy(wide_.tables_host, tiles.data(), tiles.size() * sizeof(PrefillTile));
-        wide_.tiles_at = 4 * tiles.size();
-        std::memcpy(wide_.tables_host + wide_.tiles_at, blocks.data(), blocks.size() * sizeof(PrefillBlock));
-        HM_CUDA(cudaMemcpyAsync(wide_.tables, wide_.tables_host, words * 4, cudaMemcpyHostToDevice, stream_));
+    plan->staged = most * block_bytes > wide_.kept_bytes ? wide_.own_staged : wide_.kept_staged;
+    int32_t* tables = words > WIDE_TABLE ? wide_.own_tables : wide_.kept_tables;
+    plan->tiles = reinterpret_cast<PrefillTile*>(tables);
+    plan->blocks = reinterpret_cast<PrefillBlock*>(plan->tiles + tiles.size());
+    // through pinned memory where they fit it; the copy of a larger, pageable table has read it when it returns
+    const void *from_tiles = tiles.data(), *from_blocks = blocks.data();
+    if (words <= WIDE_TABLE) {
+        uint32_t* pin = pin_u32_ + pin_u32_cap_;
+        std::memcpy(pin, tiles.data(), tiles.size() * sizeof(PrefillTile));
+        std::memcpy(pin + 4 * tiles.size(), blocks.data(), blocks.size() * sizeof(PrefillBlock));
+        from_tiles = pin;
+        from_blocks = pin + 4 * tiles.size();
     }
+    if (!tiles.empty()) HM_CUDA(cudaMemcpyAsync(plan->tiles, from_tiles, tiles.size() * sizeof(PrefillTile), cudaMemcpyHostToDevice, stream_));
+    if (!blocks.empty()) HM_CUDA(cudaMemcpyAsync(plan->blocks, from_blocks, blocks.size() * sizeof(PrefillBlock), cudaMemcpyHostToDevice, stream_));
     return HM_OK;
 }
 
 // All layers of one pass; the residual stream is left in wide_.h.
-int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches) {
+int Engine::enqueue_wide(const WidePlan& plan, const WidePass& p, const uint32_t* tokens, const int32_t* row_pos, const int32_t* row_seq, int* launches) {
     const int M = p.rows;
     const float eps = (float)cfg_.rms_norm_eps;
     cudaError_t ce = launch_embed_gather(embed_, embed_dtype_ == HM_BF16 ? 1 : 0, tokens, M, H_, V_, wide_.h, err_flag_, stream_, pdl_);
@@ -221,9 +254,9 @@ int Engine::enqueue_wide(const WidePass& p, const uint32_t* tokens, const int32_
             a.heads = heads_;
             a.scale = (float)(1.0 / std::sqrt((double)hd_));
             a.q = wide_.q;
-            a.staged = wide_.staged;
-            a.tiles = reinterpret_cast<const PrefillTile*>(wide_.tables) + g.tile0;
-            a.blocks = reinterpret_cast<const PrefillBlock*>(wide_.tables + wide_.tiles_at) + g.block0;
+            a.staged = plan.staged;
+            a.tiles = plan.tiles + g.tile0;
+            a.blocks = plan.blocks + g.block0;
             a.n_tiles = g.tiles;
             a.n_blocks = g.blocks;
             a.xp_out = wide_.att;

@@ -85,3 +85,17 @@ def test_no_copies_for_sizes_that_have_no_wide_passes(hm):
     m.prefill(synth.prompt_ids(4, 100, 512))
     assert m.wide_rows() == 0
     m.close()
+
+
+def test_a_first_long_prompt_allocates_nothing(hm):
+    # an allocation takes longer than a short prompt's wide pass saves
+    m = large(hm)
+    m.init_kv_cache(300)
+    m.prefill(synth.prompt_ids(4, 290, 512))  # kernels are loaded
+    for tokens, n in ((400, 65), (1000, 900), (250, 128)):
+        m.init_kv_cache(tokens)
+        before = free_bytes(hm)
+        m.prefill(synth.prompt_ids(5, n, 512))
+        assert m.wide_rows() == n
+        assert before - free_bytes(hm) < 2 * MB  # (what cudaMalloc hands out at least)
+    m.close()
