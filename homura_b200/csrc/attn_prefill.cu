@@ -10,7 +10,8 @@
 // contractions are warp-level MMAs (m16n8k16, f32 accumulate) on terms whose products reach 2^-24: queries and probabilities are f32 (three
 // terms each), so bf16 pages take three products and f32 pages six, the leading one in an accumulator of its own.  The sums of a 64-key block start from zero and join the
 // running result as one f32 multiply-add (the rescaling that the online softmax does anyway), so that the tensor core's truncating
-// additions never form a chain longer than a block.
+// additions never form a chain longer than a block.  Masked keys have probability zero: a value that is not finite reaches the rows of its own block of 64
+// keys in front of it too (in the decode kernels, those of its page of 16).
 // Measured: 2048 rows x 12 heads of 128 on bf16 pages 142 us (272 TFLOP/s of products), 1999 rows x 14 heads of 64 on f32 pages 126 us, bound
 // by the warp-level MMAs; the decode kernel took 32 launches of 64 rows for the same, 3500 rows of the 0.6 B geometry 113 -> 14 ms.
 #include <algorithm>
@@ -157,12 +158,14 @@ __global__ void __launch_bounds__(THREADS, (Shape<HD, BF16>::CTAS)) attn_prefill
         if (lane == 0) {
             const unsigned char* src = a.staged + ((size_t)t.block0 * a.kv.kv_heads + kvh) * (2 * S::SLOT);
             const size_t step = (size_t)a.kv.kv_heads * (2 * S::SLOT);
-            for (int i = 0; i < 2 * nb; ++i) {  // K and V of a block in turn
+            int i = 0;
+            for (; i < 2 * nb; ++i) {  // K and V of a block in turn
                 const int s = i % S::SLOTS;
                 if (i >= S::SLOTS && !mb_wait(&empty[s], ((i / S::SLOTS) & 1u) ^ 1u, a.err_flag, &s_abort)) break;
                 mb_expect_tx(&full[s], S::SLOT);
                 bulk_copy(ring + (size_t)s * S::SLOT, src + (i >> 1) * step + (i & 1) * S::SLOT, S::SLOT, &full[s]);
             }
+            mb_land_ring(full, (uint32_t)i, S::SLOTS);  // (consumers that gave up leave at once)
         }
         return;
     }

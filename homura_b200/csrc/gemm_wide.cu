@@ -72,7 +72,7 @@ __device__ __forceinline__ void tmem_wait(uint32_t (&r)[32]) {
 }
 
 struct WideShared {
-    uint64_t wfull[W_SLOTS], wempty[W_SLOTS], xfull[X_SLOTS], xempty[X_SLOTS], afull[2], aempty[2];
+    uint64_t wfull[W_SLOTS], wempty[W_SLOTS], xfull[X_SLOTS], xempty[X_SLOTS], afull[2], aempty[2], done;
     uint32_t tmem;
     volatile int abort_flag;
 };
@@ -168,6 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
         for (int s = 0; s < W_SLOTS; ++s) { mb_init(&sh.wfull[s], 1); mb_init(&sh.wempty[s], 1); }
         for (int s = 0; s < X_SLOTS; ++s) { mb_init(&sh.xfull[s], 1); mb_init(&sh.xempty[s], 1); }
         for (int s = 0; s < 2; ++s) { mb_init(&sh.afull[s], 1); mb_init(&sh.aempty[s], EPI_WARPS); }
+        mb_init(&sh.done, 1);
         sh.abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
     pdl_launch_dependents();
     if (warp != 0) pdl_wait();
 
+    uint32_t w_issued = 0, x_issued = 0;
     if (warp == 0) {
         if (lane == 0) {
             const unsigned char* W = reinterpret_cast<const unsigned char*>(a.W);
@@ -228,6 +230,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
                     }
                 }
             }
+            w_issued = max(wi, ahead);
+            x_issued = xi;
         }
     } else if (warp == 1) {
         if (lane == 0) {
@@ -345,6 +349,16 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_wide_kernel(const WideArgs a)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (sh.abort_flag) {  // a wait ran out: the copies and MMAs in flight end before the CTA does and its accumulators are freed
+        if (tid == 0) {
+            mb_land_ring(sh.wfull, w_issued, W_SLOTS);
+            mb_land_ring(sh.xfull, x_issued, X_SLOTS);
+        } else if (tid == 32) {
+            mma_commit(&sh.done);
+            mb_land(&sh.done, 0);
+        }
+        __syncthreads();
+    }
     if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 

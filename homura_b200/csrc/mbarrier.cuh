@@ -57,6 +57,16 @@ __device__ __forceinline__ bool mb_wait_limit(uint64_t* b, uint32_t parity, int*
     return true;
 }
 __device__ __forceinline__ bool mb_wait(uint64_t* b, uint32_t parity, int* err, volatile int* abort_flag) { return mb_wait_limit(b, parity, err, abort_flag, MB_SPIN_LIMIT); }
+// Bounded wait that does not look at the abort flag: what a thread has in flight (copies into shared memory, MMAs that read it) must have
+// ended before its CTA does, also where the CTA gives up.
+__device__ __forceinline__ void mb_land(uint64_t* b, uint32_t parity) {
+    for (unsigned long long it = 0; it < MB_SPIN_LIMIT && !mb_try(b, parity); ++it) {
+    }
+}
+// The same for the last `slots` of `issued` copies of a ring.
+__device__ __forceinline__ void mb_land_ring(uint64_t* full, uint32_t issued, uint32_t slots) {
+    for (uint32_t i = issued > slots ? issued - slots : 0u; i < issued; ++i) mb_land(&full[i % slots], (i / slots) & 1u);
+}
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s32(dst)), "l"(src), "r"(bytes), "r"(s32(bar)) : "memory");
 }
