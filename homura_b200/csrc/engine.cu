@@ -101,6 +101,10 @@ int Engine::create(const ModelSpec& spec, int device, bool strict_f32, Engine** 
     e->max_cluster_ = gemv_max_cluster();
     const char* notc = std::getenv("HM_NO_TC");
     e->use_tc_ = !(notc && notc[0] == '1') && !(spec.listed() && strict_f32);
+    if (const char* kb = std::getenv("HM_STAGED_KB")) {
+        e->staged_most_ = (size_t)std::max(1L, std::atol(kb)) << 10;
+        e->staged_kept_ = e->staged_most_ / 2;
+    }
     *out = e;
     return HM_OK;
 }

@@ -376,6 +376,9 @@ class Engine {
         int32_t *kept_tables = nullptr, *own_tables = nullptr;
         size_t own_words = 0;
     } wide_;
+    // Bytes of staged keys and values of one launch at most (one sequence may take more), and what is kept for them; a call that stages more
+    // takes its own (HM_STAGED_KB: other limits, for tests of launches over parts of a pass)
+    size_t staged_most_ = 512u << 20, staged_kept_ = 64u << 20;
     int wide_copies_ = -1;  // copies of quantised weights for them: not decided yet, none, all
     int wide_rows_ = 0;  // rows of the last call that ran in them
 

@@ -26,11 +26,13 @@ class Others:
         self.buffer.free()
 
 
-def load(hm, H, I, heads, kvh, layers=4, V=512):
-    """A Q8_0 model of random codes; 6 bytes per weight of copies."""
+def load(hm, H, I, heads, kvh, layers=4, V=512, dtype="Q8_0"):
+    """A model of random weights; in Q8_0 its copies take 6 bytes per weight."""
     rng = np.random.default_rng(H)
 
-    def blocks(rows, k):
+    def weights(rows, k):
+        if dtype == "BF16":
+            return synth.f32_to_bf16_rne(rng.standard_normal((rows, k), dtype=np.float32) * np.float32(0.02))
         out = np.empty((rows * k // 32, 34), np.uint8)
         out[:, :2] = np.frombuffer(np.float16(0.0005).tobytes(), np.uint8)
         out[:, 2:] = rng.integers(-60, 61, (len(out), 32), np.int8).view(np.uint8)
@@ -42,7 +44,7 @@ def load(hm, H, I, heads, kvh, layers=4, V=512):
         p = f"model.layers.{i}."
         tensors += [(p + k + "_layernorm.weight", hm.DType.BF16, (H,), one) for k in ("input", "post_attention")]
         for name, n, k in [("self_attn.q_proj", heads * hd, H), ("self_attn.k_proj", kvh * hd, H), ("self_attn.v_proj", kvh * hd, H), ("self_attn.o_proj", H, heads * hd), ("mlp.gate_proj", I, H), ("mlp.up_proj", I, H), ("mlp.down_proj", H, I)]:
-            tensors.append((p + name + ".weight", hm.DType.Q8_0, (n, k), blocks(n, k)))
+            tensors.append((p + name + ".weight", hm.DType[dtype], (n, k), weights(n, k)))
     return hm.HfModel.from_tensors(hm.TransformerConfig(H, I, heads, layers, kvh, V, 1e-6, 1e4, 32768, True, hd), tensors)
 
 
@@ -98,4 +100,18 @@ def test_a_first_long_prompt_allocates_nothing(hm):
         m.prefill(synth.prompt_ids(5, n, 512))
         assert m.wide_rows() == n
         assert before - free_bytes(hm) < 2 * MB  # (what cudaMalloc hands out at least)
+    m.close()
+
+
+def test_long_prompts_without_memory_for_their_scratch(hm):
+    m = load(hm, 1024, 4096, 16, 4, layers=2, dtype="BF16")
+    ids = synth.prompt_ids(4, 300, 512)
+    with Others(hm, 96 * MB):  # the scratch takes more than that
+        m.init_kv_cache(2048)
+        _, narrow = m.prefill(ids, want_logits=True)
+        assert m.wide_rows() == 0
+    m.reset_kv_cache()
+    _, wide = m.prefill(ids, want_logits=True)  # there is room now
+    assert m.wide_rows() == 300
+    assert np.abs(narrow - wide).max() <= 1e-4 * max(1.0, float(np.abs(wide).max()))
     m.close()

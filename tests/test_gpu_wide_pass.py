@@ -59,6 +59,47 @@ def test_mixed_runs_of_any_length(hm, oracle, name, before, rows):
     m.close()
 
 
+@pytest.mark.parametrize("kv", ["F32", "BF16"])
+@pytest.mark.parametrize("name", ["qwen2", "qwen3"])
+def test_attention_in_several_launches(hm, oracle, monkeypatch, name, kv):
+    # room for four blocks of 64 keys of f32 pages: sequences of 3, 3, 6 (more than the room by itself) and 1, each launch over the staged
+    # blocks of the one in front; and for as many bytes of bf16 pages
+    cfg, d = make_hf(name, max_position_embeddings=512)
+    block = cfg.num_key_value_heads * 2 * 3 * 64 * cfg.hd * 2
+    monkeypatch.setenv("HM_STAGED_KB", str(4 * block // 1024))
+    m = hm.HfModel.load(d)
+    m.init_kv_cache(512, batch=4, kv_dtype=hm.DType[kv])
+    before, rows = [100, 0, 300, 20], [40, 130, 60, 9]
+    ids = [synth.prompt_ids(80 + i, b + r, cfg.vocab_size) for i, (b, r) in enumerate(zip(before, rows))]
+    want = [oracle.OracleModel.from_hf_dir(d, max_seq_len=512).forward_all(t) for t in ids]
+    for i in range(4):
+        if before[i]:
+            m.step([(i, ids[i][: before[i]], [])], want_logits=False)
+    got, _, _ = m.step([(i, ids[i][before[i] :], np.arange(rows[i])) for i in range(4)], want_logits=True)
+    assert m.wide_rows() == sum(rows)
+    assert_logits_close(got, np.concatenate([w[b:] for w, b in zip(want, before)]), scale_tol=kv == "F32")
+    m.close()
+
+
+def test_tables_of_very_many_runs(hm, oracle):
+    # 600 runs of eight rows: more tiles and blocks than the kept tables hold
+    cfg, d = make_hf("qwen2", max_position_embeddings=256)
+    om = oracle.OracleModel.from_hf_dir(d, max_seq_len=64)
+    m = hm.HfModel.load(d)
+    m.init_kv_cache(32, batch=600)
+    prompts = [synth.prompt_ids(60 + i, 8, cfg.vocab_size) for i in range(7)]
+    want = []
+    for t in prompts:
+        om.reset()
+        want.append(om.forward_all(t)[-1])
+    for _ in range(2):  # taken, and again
+        m.reset_kv_cache()
+        got, _, _ = m.step([(i, prompts[i % 7], [7]) for i in range(600)], want_logits=True)
+        assert m.wide_rows() == 4800
+        assert_logits_close(got, np.stack([want[i % 7] for i in range(600)]))
+    m.close()
+
+
 def test_prompts_of_several_passes(hm, oracle):
     cfg, d = make_hf("qwen2", max_position_embeddings=4352)
     om = oracle.OracleModel.from_hf_dir(d, max_seq_len=4352)
