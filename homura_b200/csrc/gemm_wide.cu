@@ -20,9 +20,9 @@
 //     eight warps (15 us for 128 x 256 residuals, images and sums of squares; 3 us for the partial tile).
 // Measured: gate/up of 2048 rows (K 1536, N 17920) 287 us = 1.18 PFLOP/s of bf16 products, down (K 8960, N 1536) 119 + 14 us, where the
 // 64-row launches took 32 x 15.0 and 32 x 13.2 us; a prompt of 1999 tokens on the 0.5 B stack 52.1 -> 9.2 ms,
-// 1021 tokens on TinyLlama Q8_0 60.1 -> 12.1 ms and Q4_0 66.8 -> 10.7 ms (64-row launches on digit planes and integer MMAs before).  What bounds it is the
-// traffic between L2 and shared memory (80 KB per k-block and SM) and the read-back of the accumulators: one per two k-blocks costs 12 %
-// against one per four, which leaves 1.8 times the error.
+// 1021 tokens on TinyLlama Q8_0 60.1 -> 12.1 ms and Q4_0 66.8 -> 10.7 ms (64-row launches on digit planes and integer MMAs before).  By the sizes (no counter
+// was taken) the traffic between L2 and shared memory bounds it (80 KB per k-block and SM), and the read-back of the accumulators: one per two k-blocks costs
+// 12 % against one per four, which leaves 1.8 times the error.
 #include <algorithm>
 #include <type_traits>
 
