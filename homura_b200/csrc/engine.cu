@@ -1519,6 +1519,7 @@ int Engine::prefill(int seq, const int64_t* ids, int n, float* logits, uint32_t*
     float* land = logits ? logits_landing(logits, (size_t)V_ * 4) : nullptr;
     if (logits) HM_CUDA(cudaMemcpyAsync(land, logits_, (size_t)V_ * 4, cudaMemcpyDeviceToHost, stream_));
     if (int qrc = queue_error_copy()) return qrc;
+    if (logits && land != logits) touch_out(logits, (size_t)V_ * 4, stream_);
     HM_CUDA(cudaStreamSynchronize(stream_));
     int rc = check_device_error();
     if (rc) return rc;
@@ -1555,6 +1556,7 @@ int Engine::decode_step(const uint32_t* tokens, float* logits, uint32_t* next_to
     HM_CUDA(cudaMemcpyAsync(pin_u32_ + batch_, next_dev_, (size_t)batch_ * 4, cudaMemcpyDeviceToHost, stream_));
     if (logits && !graph_exec_host_) HM_CUDA(cudaMemcpyAsync(land, logits_, (size_t)batch_ * V_ * 4, cudaMemcpyDeviceToHost, stream_));
     if (int qrc = queue_error_copy()) return qrc;
+    if (logits && land != logits) touch_out(logits, (size_t)batch_ * V_ * 4, stream_);
     HM_CUDA(cudaStreamSynchronize(stream_));
     {
         int erc = check_device_error();
@@ -1893,6 +1895,7 @@ int Engine::decode_step_sampled(const uint32_t* tokens, const hm_sampling* sp, u
     if (logits) HM_CUDA(cudaMemcpyAsync(land, logits_, B * V_ * 4, cudaMemcpyDeviceToHost, stream_));
     rc = queue_error_copy();
     if (rc) return rc;
+    if (logits && land != logits) touch_out(logits, B * V_ * 4, stream_);
     HM_CUDA(cudaStreamSynchronize(stream_));
     rc = check_device_error();
     if (rc) return rc;
