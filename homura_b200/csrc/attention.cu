@@ -348,8 +348,10 @@ __device__ __forceinline__ void merge_slots_and_write(const AttnArgs& a, int nsu
     if (tid == 0) a.tickets[m * a.kv_heads + kvh] = 0u;
 }
 
+// The cluster variants of 128-wide heads may take 128 registers: left to itself the compiler keeps them at 80 and spills, and a launch with a stack
+// costs the chain that it is part of 8 us (1.5 B, one sequence on bf16 pages: 1.54 -> 1.16 ms per step).
 template <int HD, bool BF16, bool CL>
-__global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(ATT_THREADS, CL && HD == 128 ? 2 : 0) attn_decode_kernel(const AttnArgs a) {
     using TL = Tile<HD, BF16>;
     using T = typename std::conditional<BF16, uint16_t, float>::type;
     constexpr int EPL = HD / 32;  // output elements per lane

@@ -215,11 +215,9 @@ __device__ __forceinline__ void merge_stage(const GemvExt& a, float* __restrict_
     __syncthreads();  // part is written again behind the multiply
 }
 
-// The unsplit M = 1 variant (LM head: one long stream per CTA) runs three CTAs per SM (<= 85
-// registers) to keep ~96 KB of weight loads in flight per SM; measured 5.0 -> 5.3 TB/s.  The
-// clustered one-row variants are latency chains and were slower under a tighter register budget.  The
-// 2- and 4-row variants (split or not) are held to 128 registers so that two CTAs stay resident per SM:
-// wide projections launch more CTAs than there are SMs.
+// The variants of up to four rows (split or not) are held to 128 registers, so that two CTAs stay resident per SM: wide projections launch more
+// CTAs than there are SMs.  (Three CTAs per SM of the unsplit one-row variant, the LM head, spill at 80 registers: a step of the 0.6 B stack 0.650 ms with two
+// and 0.664 with three, of the 0.5 B and 1.5 B stacks the same.)
 // ST (with CL): the CTA's whole weight slice (rows [k0, k0+nrows) of its slab, one contiguous byte range of
 // at most GEMV_STAGE_MAX bytes) is pulled into shared memory by bulk copies issued BEFORE the dependency
 // wait, so that by the time the predecessor has finished the multiply runs out of shared memory and HBM
@@ -228,7 +226,7 @@ template <int X>
 using GemvArgsOf = typename std::conditional<X == 2, GemvArgs, typename std::conditional<X == 1, GemvExt, GemvBase>::type>::type;
 
 template <int M, bool CL, bool ST, int X>
-__global__ void __launch_bounds__(GEMV_THREADS, CL ? (M <= 4 ? 2 : 1) : (M == 1 ? 3 : (M <= 4 ? 2 : 1))) gemv_bf16_kernel(const GemvArgsOf<X> a) {
+__global__ void __launch_bounds__(GEMV_THREADS, M <= 4 ? 2 : 1) gemv_bf16_kernel(const GemvArgsOf<X> a) {
     extern __shared__ __align__(128) float smem_raw[];
     const int rps = a.rows_per_split;
     // staged weights first (bulk copies want 16-byte aligned destinations), then the f32 scratch
