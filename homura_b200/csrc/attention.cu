@@ -35,8 +35,7 @@ constexpr int ATT_WARPS = 8;
 constexpr int ATT_THREADS = ATT_WARPS * 32;
 constexpr int G_MAX = 8;   // query heads per KV head handled by one CTA
 constexpr int MAXP = 4;    // 16-byte pieces of K (and of V) a thread may hold in flight
-constexpr int ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used
-constexpr int RES_MAX_PAGES = 8;  // decode launches with at most this many pages per CTA keep all of them in shared memory
+constexpr int ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used (in clusters: see launch_tc)
 
 template <int HD, bool BF16>
 struct Tile {
@@ -55,13 +54,13 @@ __host__ __device__ inline int pick_nsub(int g) {
 }
 
 // Page slots of the short-context kernel: nsub slots reused group after group, or -- when a decode
-// launch gives a CTA at most RES_MAX_PAGES pages -- one slot per page, so that every page that is
+// launch gives a CTA at most early_pages - 1 pages -- one slot per page, so that every page that is
 // final before the dependency wait is already in shared memory when the wait returns.
 template <int HD, bool BF16>
 __host__ __device__ inline int pick_nslots(int g, int early_pages, int max_pages, int nsplit) {
     const int nsub = pick_nsub<HD, BF16>(g);
     const int cap = (max_pages + nsplit - 1) / nsplit;
-    if (early_pages < 2 || cap > RES_MAX_PAGES) return nsub;
+    if (early_pages < 2 || cap > early_pages - 1) return nsub;
     return (cap + nsub - 1) / nsub * nsub;
 }
 
@@ -1005,8 +1004,16 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     const int g = a.heads / a.kv_heads;
     const int pages_per_cta = (a.max_pages + a.nsplit - 1) / a.nsplit;
     // long contexts: the bulk-copy ring; a slot layout needs ATT_WARPS / g >= 1 as in the kernel above
-    const bool stream = a.stream_pages > 0 && pages_per_cta >= ST_MIN_PAGES && pages_per_cta <= ST_MAX_PT;
     const int slots = CL ? merge_slot_cap(a.nsplit) : 1;  // rank 0 of a cluster receives every split's triples
+    const long ctas = (long)a.nsplit * a.kv_heads * M;
+    // A cluster's CTAs need as many SMs of one GPC at the same time: more than four clusters of sixteen want to share SMs.
+    const bool crowd = CL && ctas > 64;
+    // Pages per CTA from which it streams.  In clusters it merges by asynchronous stores as well and soon wins: 1.5 B with 1000 tokens (four pages) 1.29 -> 1.22 ms
+    // per step, bf16 pages 1.30 -> 1.16; TinyLlama Q8_0 0.67 -> 0.65 and 0.61; two sequences of the 0.5 B stack with 900 0.66 -> 0.61.  One sequence on two
+    // 64-wide KV heads, 32 CTAs, from seven on (0.5 B: four pages 0.56 and 0.60, eight 0.65 and 0.63); CTAs that cannot share an SM from five on (0.6 B, f32
+    // pages: three 0.71 and 0.75, five 0.77 and 0.76; four sequences of 1.5 B on bf16 pages: four 1.71 and 1.77).
+    const int from = !CL ? ST_MIN_PAGES : HD == 64 && ctas <= 32 ? 7 : crowd && 2 * stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, StTile<HD, BF16>::STAGES) > 227 * 1024 ? 5 : 3;
+    const bool stream = a.stream_pages > 0 && pages_per_cta >= from && pages_per_cta <= ST_MAX_PT;
     // The ring bounds what one CTA keeps in flight (a warp asks for its next page only when it has freed a stage).
     // Launches that leave every CTA an SM to itself (64 sequences x 2 KV heads, one split: 128 CTAs) get as deep a
     // ring as shared memory holds, in multiples of the eight consumer warps; larger launches keep two CTAs per SM.
@@ -1015,7 +1022,7 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     if (stream) {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if ((long)a.nsplit * a.kv_heads * M <= sms) {
+        if (ctas <= sms && !crowd) {
             const int want = std::min(ST_MAX_STAGES, (pages_per_cta + ATT_WARPS - 1) / ATT_WARPS * ATT_WARPS);
             while (stages + ATT_WARPS <= want && stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, stages + ATT_WARPS) <= 216 * 1024) stages += ATT_WARPS;
         }

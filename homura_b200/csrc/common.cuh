@@ -496,7 +496,7 @@ struct AttnArgs {
     unsigned char* xp_out;  // optional: write the output as packed tensor-core activations (tc_xpack_store) instead of `out`
     int xp_mpad;
     int early_pages;     // >= 1: every row is its own sequence (decode), so the pages below the one of the new token may be read before the dependency wait;
-                         // 2: and every page of a split gets its own shared-memory slot (small launches, where latency counts and occupancy does not)
+                         // n >= 2: and the pages of a split of at most n - 1 get a shared-memory slot each
     int stream_pages;    // > 0: long contexts may use the bulk-copy ring variant (pages per CTA decided from max_pages / nsplit)
     int st_stages;       // stages of that variant's page ring, a multiple of its 8 consumer warps (filled in by the launcher)
     int* err_flag;       // raised to 2 when a bounded wait of that variant runs out

@@ -357,7 +357,9 @@ class Engine {
     float *att_acc_ = nullptr, *att_ml_ = nullptr;
     unsigned int* att_tickets_ = nullptr;
     int att_nsplit_ = 1;
+    int att_spread_ = 1;  // splits of a decode pass that also asks for weights (kv_alloc)
     bool att_cluster_ = true;
+    bool att_decode_cluster_ = true;  // of decode passes
     int* err_flag_ = nullptr;
     unsigned int* fin_ticket_ = nullptr;  // ticket of the LM head's folded argmax
 
