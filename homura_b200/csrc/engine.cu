@@ -524,6 +524,13 @@ int Engine::ensure_scratch(int rows) {
     return HM_OK;
 }
 
+// Weights that a launch of a step of few rows asks the L2 for, at most.  More of them is memory traffic that the launches in between wait for, and an SM asks for
+// 0.33 MB per microsecond at most (the attention of a cache of two pages is four CTAs: 0.5 B, 17 MB, 22 tokens 0.80 and 0.48 ms per step); ms with
+// the attention asking for all of gate/up and the projections for all of theirs, with none, and with 4 and 8 MB: 1.5 B, one sequence 1.16, 1.04, 1.02 (2000 tokens
+// 1.23, 1.14, 1.10), two 1.32, 1.16, 1.15, four 1.55, 1.51, 1.50; 0.5 B, one 0.492, 0.485, 0.475 (2000 tokens 0.627, 0.592, 0.586), four 0.716, 0.723,
+// 0.715; 0.6 B, one 0.643, 0.634, 0.642, two 0.859, 0.840, 0.845.
+static constexpr size_t ATTN_PF = 4u << 20, PROJ_PF = 8u << 20;
+
 // ---- KV cache --------------------------------------------------------------------------------
 
 int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, long pool_tokens) {
@@ -623,18 +630,8 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     const long pairs = (long)batch * kvh_;
     const int reach = pairs <= 4 ? 256 : pairs <= 8 ? (kv_bf16_ || hd_ == 64 ? 256 : 80) : 64;
     att_decode_cluster_ = use_clusters_ && max_pages_ <= reach && pairs < sm_count_ / 2;
-    const int by_pages = attn_pick_cluster(max_pages_, std::min(max_cluster_, 16));
-    att_nsplit_ = att_cluster_ ? by_pages : std::max(att_decode_cluster_ ? by_pages : 1, attn_pick_nsplit(batch, kvh_, max_pages_, sm_count_, kv_bf16_));
-    // Decode passes of few rows prefetch the gate/up weights from the attention launch, and an SM asks the L2 for 0.33 MB per microsecond at most: a cache of two
-    // pages, whose launch would be four CTAs, waited 13 us per layer for 17 MB.  Splits without a page are CTAs that only ask.  One for every 0.8 MB,
-    // as 2 to 4, 8 or 16 (the sizes that their merge knows); steps of one sequence in a cache of 22 tokens, ms with a split per page and so: 0.5 B 0.80 and 0.49,
-    // 1.5 B 2.45 and 1.17, of four 1.77 and 1.55; 0.6 B, whose eight KV heads ask for 12.6 MB, keeps a split per page (0.62; 0.68 with 16).  No weights
-    // are asked for from quantised models' launches (TinyLlama Q8_0 0.555; 0.592 with 16).
-    att_spread_ = att_decode_cluster_ ? by_pages : att_nsplit_;
-    if (att_decode_cluster_ && use_prefetch_ && !quant_ && !spec_.listed()) {
-        const int want = (int)std::min<uint64_t>(16, layers_[0].gu.bytes() / ((uint64_t)batch * kvh_ * 800000));
-        att_spread_ = std::max(by_pages, std::min(want <= 4 ? want : want <= 8 ? 8 : 16, std::min(max_cluster_, 16)));
-    }
+    att_by_pages_ = attn_pick_cluster(max_pages_, std::min(max_cluster_, 16));
+    att_nsplit_ = att_cluster_ ? att_by_pages_ : std::max(att_decode_cluster_ ? att_by_pages_ : 1, attn_pick_nsplit(batch, kvh_, max_pages_, sm_count_, kv_bf16_));
     if (!spec_.listed()) {
         HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * hd_ * 4));
         HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * 2 * 4));
@@ -1135,7 +1132,7 @@ AttnArgs Engine::attn_args(int l, int M, const float* q, const int32_t* row_pos,
     // fewer splits when the rows alone fill the SMs: about two CTAs per SM on the cluster path (caches
     // of up to 1024 tokens), the kernel's cost model on the long-context path
     const bool decode = row_seq == nullptr, cluster = decode ? att_decode_cluster_ : att_cluster_;
-    at.nsplit = std::min(decode && cluster && !tall_rows(M) ? att_spread_ : att_nsplit_, cluster ? std::min(std::max(1, (2 * sm_count_ + M * kvh_ - 1) / (M * kvh_)), 16) : attn_pick_nsplit(M, kvh_, max_pages_, sm_count_, kv_bf16_));
+    at.nsplit = std::min(cluster ? att_by_pages_ : att_nsplit_, cluster ? std::min(std::max(1, (2 * sm_count_ + M * kvh_ - 1) / (M * kvh_)), 16) : attn_pick_nsplit(M, kvh_, max_pages_, sm_count_, kv_bf16_));
     at.cluster = cluster ? 1 : 0;
     at.stream_pages = 1;
     // Decode passes: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs per SM may keep the pages
@@ -1202,7 +1199,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
         pf_bytes_ = 0;
         if (!pf || !w || !w->slabs || off >= w->bytes()) return;
         pf_ptr_ = (const char*)w->slabs + off;
-        pf_bytes_ = std::min(cap, w->bytes() - off);
+        pf_bytes_ = std::min(cap, std::min(PROJ_PF, w->bytes() - off));
     };
     constexpr size_t LM_PF = 24u << 20;  // the LM head does not fit the L2: only its first 2 x 24 MB are fetched early
     int rc;
@@ -1254,7 +1251,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
 #endif
         if (pf) {
             at.pf_ptr = w.gu.slabs;
-            at.pf_bytes = w.gu.bytes();
+            at.pf_bytes = std::min<uint64_t>(w.gu.bytes(), ATTN_PF);
         }
         if (want(PC_ATTN)) {
             ce = launch_attn_decode(at, M, kv_bf16_, stream_, pdl_);

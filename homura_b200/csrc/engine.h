@@ -357,7 +357,7 @@ class Engine {
     float *att_acc_ = nullptr, *att_ml_ = nullptr;
     unsigned int* att_tickets_ = nullptr;
     int att_nsplit_ = 1;
-    int att_spread_ = 1;  // splits of a decode pass that also asks for weights (kv_alloc)
+    int att_by_pages_ = 1;  // splits of a cluster
     bool att_cluster_ = true;
     bool att_decode_cluster_ = true;  // of decode passes
     int* err_flag_ = nullptr;
