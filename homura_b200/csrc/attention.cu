@@ -665,6 +665,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
     const int g = a.heads / a.kv_heads;
     const int head0 = kvh * g;
 
+    if (CL) cluster_arrive_release();  // waited for in front of the merge: nobody stores into a CTA that has not started
     if (tid == 0) {
         for (int s = 0; s < NST; ++s) {
             mb_init(&full[s], 1);
@@ -984,6 +985,7 @@ __global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnAr
         }
     }
     __syncthreads();
+    if (CL) cluster_wait_acquire();
     merge_slots_and_write<HD, CL>(a, ST::CW, g, head0, split, kvh, m, w_ml, w_acc, c_o, c_ml, &s_last);
 }
 
