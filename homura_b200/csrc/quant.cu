@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(QT, (M == 1 && ST) ? 3 : 1) gemv_quant_kernel(
     HM_TRACE(if (tr) a.trace[0] = global_timer();)
     HM_TRACE(if (a.trace && tid == 0) atomicMax(a.trace + 8, global_timer());)
     pdl_launch_dependents();
+    if (CL) cluster_arrive_release();  // waited for in front of the stores into rank 0: it has started by then
 
     // weights never depend on a previous kernel: the whole slice into shared memory (ST), or the first batch of
     // streaming loads into registers, before the dependency wait
@@ -480,6 +481,7 @@ __global__ void __launch_bounds__(QT, (M == 1 && ST) ? 3 : 1) gemv_quant_kernel(
         // every rank pushes its partial into rank 0's shared memory, arrives at the cluster barrier and is
         // done; rank 0 waits once and adds the slots in rank order from its own memory
         float* slots = red + 8 * M * 32;  // [ksplit][M][32]
+        cluster_wait_acquire();
         if (tid < M * 32) {
             if (split == 0) slots[tid] = v;
             else st_dsmem_f32(dsmem_addr(slots + split * (M * 32) + tid, 0u), v);
@@ -701,6 +703,7 @@ __global__ void __launch_bounds__(QT) gemm_quant_kernel(const QuantArgs a) {
     const int kb0 = split * a.kb_per_split, kb1 = min(nb, kb0 + a.kb_per_split);
     const int nkb = max(0, kb1 - kb0);
     pdl_launch_dependents();
+    if (CL) cluster_arrive_release();  // waited for in front of the stores into rank 0: it has started by then
     // the tile's codes and scales do not depend on the launch in front: staged before the dependency wait, in pieces
     const int ck = max(8, ((nkb + NCHUNK - 1) / NCHUNK + 7) / 8 * 8);
     if (tid == 0) {
@@ -826,6 +829,7 @@ __global__ void __launch_bounds__(QT) gemm_quant_kernel(const QuantArgs a) {
     __syncthreads();
     if (CL) {
         // every rank pushes its sums into rank 0's slots and is done; rank 0 adds them in rank order
+        cluster_wait_acquire();
         if (alias) cluster_sync_all();  // nobody reads staged codes any more: the slots may overwrite them
         for (int t = tid; t < GR * 32; t += QT) {
             if (split == 0) slots[t] = vals[t];
