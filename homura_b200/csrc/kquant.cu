@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(KT) gemv_kquant_kernel(const KQuantArgs a) {
     const int npieces = ttype == 2 ? 13 : 9;
 
     pdl_launch_dependents();
+    if (CL) cluster_arrive_release();  // waited for in front of the stores into rank 0: it has started by then
     // weights never depend on the previous kernel: ask the L2 for this CTA's super-blocks before the dependency wait
     // (a Q4_K tile fills 9 of its slot's 13 pieces and no scale words: only the bytes that will be read are asked for)
     if (ttype != 0) {
@@ -495,6 +496,7 @@ __global__ void __launch_bounds__(KT) gemv_kquant_kernel(const KQuantArgs a) {
         // every rank pushes its partial into rank 0's shared memory, arrives at the cluster barrier and is
         // done; rank 0 waits once and adds the slots in rank order from its own memory
         float* slots = red + 8 * M * 32;  // [ksplit][M][32]
+        cluster_wait_acquire();
         if (tid < M * 32) {
             if (split == 0) slots[tid] = v;
             else st_dsmem_f32(dsmem_addr(slots + split * (M * 32) + tid, 0u), v);

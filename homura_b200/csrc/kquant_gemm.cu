@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(KT) gemm_q4k_kernel(const KQuantArgs a) {
     __shared__ volatile int s_abort;
     const unsigned char* tbase = a.data + ((size_t)tile * nb + kb0) * KQ_SLOT_BYTES;
     pdl_launch_dependents();
+    if (CL) cluster_arrive_release();  // waited for in front of the stores into rank 0: it has started by then
     // the tile's slots do not depend on the launch in front: staged before the dependency wait, in up to four pieces
     const int ck = max(1, (nkb + NCHUNK - 1) / NCHUNK);
     if (tid == 0) {
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(KT) gemm_q4k_kernel(const KQuantArgs a) {
             for (int c = 0; c < 2; ++c) vals[(8 * warp + 2 * q + c) * 32 + 16 * rg + 8 * rs + g] = acc[rg][rs][c];
     __syncthreads();
     if (CL) {
+        cluster_wait_acquire();
         if (alias) cluster_sync_all();  // nobody reads staged slots any more: the receive slots may overwrite them
         for (int t = tid; t < GR * 32; t += KT) {
             if (split == 0) slots[t] = vals[t];

@@ -6,7 +6,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "homura_b200", "csrc")
-FILES = ["attention.cu", "gemm_tc.cu", "gemv_kernel.cuh", "gla.cuh", "gqa_attn.cu", "gqa_talk.cuh", "moe.cu", "quant.cu", "recur.cu", "sampler.cu"]
+FILES = ["attention.cu", "gemm_tc.cu", "gemv_kernel.cuh", "gla.cuh", "gqa_attn.cu", "gqa_talk.cuh", "kquant.cu", "kquant_gemm.cu", "moe.cu", "quant.cu", "recur.cu", "sampler.cu"]
 PRIMITIVE = re.compile(r"\b(?:st_dsmem|st_async|red_dsmem)_\w+\(")
 # (one behind a condition counts where the condition says that there is a cluster)
 BARRIER = re.compile(r"(?<!\) )(?:if \((?:CL|\w+ > 1)\) )?\bcluster_(?:wait_acquire|sync_all)\(\)")
