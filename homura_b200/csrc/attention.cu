@@ -23,6 +23,7 @@
 
 #include <algorithm>
 
+#include "attn_plan.h"
 #include "common.cuh"
 #include "launch_attrs.h"
 #include "mbarrier.cuh"
@@ -35,7 +36,6 @@ constexpr int ATT_WARPS = 8;
 constexpr int ATT_THREADS = ATT_WARPS * 32;
 constexpr int G_MAX = 8;   // query heads per KV head handled by one CTA
 constexpr int MAXP = 4;    // 16-byte pieces of K (and of V) a thread may hold in flight
-constexpr int ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used (in clusters: see launch_tc)
 
 template <int HD, bool BF16>
 struct Tile {
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CL && HD == 128 ? 2 : 0) attn_dec
 // chunk-major K tile makes that read conflict-free while the query chunk is a broadcast), and a V row
 // is read once per token for g heads.  That cuts shared-memory traffic per page by about 3x against
 // one-warp-per-head, which is what bounds the kernel above on long contexts.  Used when a CTA has at
-// least ST_MIN_PAGES pages to read.
+// least ATT_ST_MIN_PAGES pages to read.
 constexpr int ST_THREADS = ATT_THREADS + 32;
 constexpr int ST_MAX_STAGES = 24;
 constexpr int ST_RING_BYTES = 64 * 1024;  // per CTA; two CTAs per SM keep 128 KB of pages in flight
@@ -1014,7 +1014,7 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     // per step, bf16 pages 1.30 -> 1.16; TinyLlama Q8_0 0.67 -> 0.65 and 0.61; two sequences of the 0.5 B stack with 900 0.66 -> 0.61.  One sequence on two
     // 64-wide KV heads, 32 CTAs, from seven on (0.5 B: four pages 0.56 and 0.60, eight 0.65 and 0.63); CTAs that cannot share an SM from five on (0.6 B, f32
     // pages: three 0.71 and 0.75, five 0.77 and 0.76; four sequences of 1.5 B on bf16 pages: four 1.71 and 1.77).
-    const int from = !CL ? ST_MIN_PAGES : HD == 64 && ctas <= 32 ? 7 : crowd && 2 * stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, StTile<HD, BF16>::STAGES) > 227 * 1024 ? 5 : 3;
+    const int from = !CL ? ATT_ST_MIN_PAGES : HD == 64 && ctas <= 32 ? 7 : crowd && 2 * stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, StTile<HD, BF16>::STAGES) > 227 * 1024 ? 5 : 3;
     const bool stream = a.stream_pages > 0 && pages_per_cta >= from && pages_per_cta <= ST_MAX_PT;
     // The ring bounds what one CTA keeps in flight (a warp asks for its next page only when it has freed a stage).
     // Launches that leave every CTA an SM to itself (64 sequences x 2 KV heads, one split: 128 CTAs) get as deep a
@@ -1089,51 +1089,6 @@ cudaError_t launch_t(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
 }
 
 }  // namespace
-
-// Enough (row, KV head, split) CTAs to cover the SMs about twice, at least two pages each.
-int attn_pick_nsplit(int M, int kv_heads, int max_pages, int sm_count, bool bf16_pages) {
-    // Splits per (row, KV head): minimise waves x (fixed cost per CTA + pages per CTA) + merge cost.
-    // Units are "pages streamed by one CTA": the fixed cost (launch, query and page-table loads) is
-    // worth about eight pages, merging one more partial about half a page.  The streaming variant
-    // (>= ST_MIN_PAGES pages per CTA) keeps two CTAs per SM resident, the short-context kernel four.
-    // max_pages is the capacity the launch is sized for (a captured graph cannot follow the length).
-    const long pairs = (long)M * kv_heads;
-    int cap = (max_pages + 1) / 2;  // at least two pages per split
-    if (cap > sm_count) cap = sm_count;
-    if (cap < 1) cap = 1;
-    int best = 1;
-    long best_cost = -1;
-    for (int n = 1; n <= cap; ++n) {
-        const int ppc = (max_pages + n - 1) / n;
-        const bool streaming = ppc >= ST_MIN_PAGES;
-        const long slots = (streaming ? 2L : 4L) * sm_count;
-        const long waves = (pairs * n + slots - 1) / slots;
-        // doubled so that the half page per partial stays an integer; a page costs the short-context
-        // kernel about twice what it costs the streaming one (every query head re-reads the tile)
-        // having any split at all costs a round trip of the partial triples through global memory, a ticket and a
-        // second merge by the last CTA: about twenty pages' worth (64 sequences at 36 pages: one split 15.4 us, two 17.1)
-        // a streaming launch that leaves every CTA an SM to itself gets the deep page ring (launch_tc), which about
-        // halves what a page costs its CTA while the cache is short (measured on bf16 pages: 64 x 2 CTAs at 43 pages, one
-        // split 11.9 us, two 18.7); on long caches two CTAs per SM stream faster than one with a deep ring, and on f32
-        // pages fewer splits lost at every length
-        const bool deep = streaming && bf16_pages && max_pages <= 64 && pairs * n <= sm_count;
-        const long cost = 2 * waves * (8 + (streaming ? ppc : 2 * ppc)) / (deep ? 2 : 1) + (deep ? 8 : 0) + n + (n > 1 ? 40 : 0);
-        if (best_cost < 0 || cost < best_cost) {
-            best_cost = cost;
-            best = n;
-        }
-    }
-    return best;
-}
-
-// Cluster variant: the splits of a (row, KV head) form one cluster; one page per CTA when the
-// context allows, at most max_cluster CTAs.
-int attn_pick_cluster(int max_pages, int max_cluster) {
-    int n = max_pages;
-    if (n > max_cluster) n = max_cluster;
-    if (n < 1) n = 1;
-    return n;
-}
 
 cudaError_t launch_attn_decode(const AttnArgs& a, int M, bool kv_bf16, cudaStream_t st, bool pdl) {
     if (a.page_tokens != PT || a.heads % a.kv_heads != 0 || a.heads / a.kv_heads > G_MAX) return cudaErrorInvalidValue;

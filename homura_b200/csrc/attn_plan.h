@@ -1,0 +1,102 @@
+// How the attention launches of steps and small passes over the paged cache are cut (attention.cu).  Host only and free of CUDA.
+#pragma once
+#include <algorithm>
+
+namespace hm {
+
+constexpr int ATT_ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used (in clusters: see launch_tc)
+
+// Splits per (row, KV head) through global scratch: minimise waves x (fixed cost per CTA + pages per CTA) + merge cost.
+// Units are "pages streamed by one CTA": the fixed cost (launch, query and page-table loads) is
+// worth about eight pages, merging one more partial about half a page.  The streaming variant
+// (>= ATT_ST_MIN_PAGES pages per CTA) keeps two CTAs per SM resident, the short-context kernel four.
+// max_pages is the capacity the launch is sized for (a captured graph cannot follow the length).
+inline int attn_pick_nsplit(int M, int kv_heads, int max_pages, int sm_count, bool bf16_pages) {
+    const long pairs = (long)M * kv_heads;
+    int cap = (max_pages + 1) / 2;  // at least two pages per split
+    if (cap > sm_count) cap = sm_count;
+    if (cap < 1) cap = 1;
+    int best = 1;
+    long best_cost = -1;
+    for (int n = 1; n <= cap; ++n) {
+        const int ppc = (max_pages + n - 1) / n;
+        const bool streaming = ppc >= ATT_ST_MIN_PAGES;
+        const long slots = (streaming ? 2L : 4L) * sm_count;
+        const long waves = (pairs * n + slots - 1) / slots;
+        // doubled so that the half page per partial stays an integer; a page costs the short-context
+        // kernel about twice what it costs the streaming one (every query head re-reads the tile)
+        // having any split at all costs a round trip of the partial triples through global memory, a ticket and a
+        // second merge by the last CTA: about twenty pages' worth (64 sequences at 36 pages: one split 15.4 us, two 17.1)
+        // a streaming launch that leaves every CTA an SM to itself gets the deep page ring (launch_tc), which about
+        // halves what a page costs its CTA while the cache is short (measured on bf16 pages: 64 x 2 CTAs at 43 pages, one
+        // split 11.9 us, two 18.7); on long caches two CTAs per SM stream faster than one with a deep ring, and on f32
+        // pages fewer splits lost at every length
+        const bool deep = streaming && bf16_pages && max_pages <= 64 && pairs * n <= sm_count;
+        const long cost = 2 * waves * (8 + (streaming ? ppc : 2 * ppc)) / (deep ? 2 : 1) + (deep ? 8 : 0) + n + (n > 1 ? 40 : 0);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = n;
+        }
+    }
+    return best;
+}
+
+// One launch: splits of a (row, KV head), and whether they are a cluster.
+struct AttnCut {
+    int nsplit;
+    bool cluster;
+    int early_pages;  // AttnArgs::early_pages
+};
+
+// What a cache's shape decides (made with the cache), and what a launch of M rows adds to it.
+struct AttnPlan {
+    int kvh = 1, hd = 64, max_pages = 1, sms = 148;
+    bool bf16 = false;
+    int by_pages = 1;             // splits of a cluster: a page each while the cache is short
+    int batch_splits = 1;         // of a pass of as many rows as there are sequences through global scratch
+    bool cluster = false;         // passes with several rows of a sequence (prompt chunks, mixed batches)
+    bool decode_cluster = false;  // steps: a row per sequence
+
+    AttnPlan() = default;
+    AttnPlan(int batch, int kvh_, int hd_, bool bf16_, int pages, int sm_count, bool use_clusters, int max_cluster) : kvh(kvh_), hd(hd_), max_pages(pages), sms(sm_count), bf16(bf16_) {
+        const long pairs = (long)batch * kvh;
+        by_pages = std::max(1, std::min(pages, std::min(max_cluster, 16)));
+        batch_splits = attn_pick_nsplit(batch, kvh, pages, sms, bf16);
+        // up to 1024 tokens of capacity the splits of a (row, KV head) are one cluster of at most 16 CTAs, one page
+        // per split while the context allows (a page is about 0.65 us of dependent instructions, so pages of a
+        // split cost more than the wider merge); longer caches need more CTAs than a cluster holds and merge
+        // through global scratch + ticket
+        // ... and only while the (row, KV head) pairs alone do not fill the GPU: with half an SM's worth of pairs or more
+        // the launch is a throughput problem (64 sequences stream 39 MB of pages per layer), which the cost model
+        // of attn_pick_nsplit answers with few splits of many pages each, i.e. the bulk-copy ring kernel
+        cluster = use_clusters && pages <= 64 && pairs < sms / 2;
+        // Decode passes of few (row, KV head) pairs stay clusters of sixteen CTAs on longer caches too (the streaming kernel from a few pages per CTA on, launch_tc): ms per
+        // step with splits through global scratch and so, 1.5 B with 1200 tokens 1.62 and 1.23, 2000 1.63 and 1.25 (bf16 pages 1.48 and 1.17), 4000 1.53 and
+        // 1.38; 0.5 B 1200 0.79 and 0.59, 4000 0.71 and 0.63; TinyLlama Q8_0 2000 0.76 and 0.67; two sequences of 1.5 B, 1500 1.70 and 1.29.  Eight pairs are 128 CTAs,
+        // which must share SMs to be eight clusters at once: f32 pages of 128-wide heads do not fit twice (0.6 B with 2000 0.76 and 0.79, 4000 0.81 and 0.96).
+        const int reach = pairs <= 4 ? 256 : pairs <= 8 ? (bf16 || hd == 64 ? 256 : 80) : 64;
+        decode_cluster = use_clusters && pages <= reach && pairs < sms / 2;
+    }
+
+    // Splits that the scratch of a row must hold: of every launch that goes through it.
+    int scratch_splits() const { return cluster || decode_cluster ? std::max(by_pages, batch_splits) : batch_splits; }
+
+    AttnCut cut(int M, bool decode) const {
+        AttnCut c;
+        c.cluster = decode ? decode_cluster : cluster;
+        // Fewer splits where the rows alone fill the SMs: about two CTAs per SM in clusters, the kernel's cost model otherwise.  The model knows neither
+        // that the rows of a prompt share their pages nor what the merge of so many partials costs: it is held to the splits of a step (a 40-row chunk
+        // behind 1500 tokens of the 1.5 B shapes, bf16 pages: 77 us per layer with the step's 7 splits at most, 143 with the 16 of its clusters).
+        c.nsplit = c.cluster ? std::min(by_pages, std::max(1, (2 * sms + M * kvh - 1) / (M * kvh))) : std::min(batch_splits, attn_pick_nsplit(M, kvh, max_pages, sms, bf16));
+        // Decode passes: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs per SM may keep the pages
+        // of a split (eight at most) in slots of their own, which takes the loads in front of the wait; but shared memory keeps the next projection's CTAs, whose
+        // weights arrive meanwhile, off those SMs.  One page per split only where the launch is 32 CTAs or, with 128-wide heads, more than 64: ms per step with up
+        // to eight and so, one sequence, 1.5 B with 600 tokens 1.47 and 1.24, 0.5 B with 1000 0.66 and 0.56, 0.6 B with 1000 0.77 and 0.74; four sequences of 1000,
+        // 1.5 B 2.00 and 1.69; elsewhere the other way round, 0.5 B, four of 1000 (64-wide heads) 0.80 and 0.82, 1.5 B, two of 800 (64 CTAs) 1.36 and 1.43.
+        const long ctas = (long)M * kvh * c.nsplit;
+        c.early_pages = !decode ? 0 : ctas > 2L * sms ? 1 : ctas <= 32 || (hd == 128 && ctas > 64) ? 2 : 9;
+        return c;
+    }
+};
+
+}  // namespace hm

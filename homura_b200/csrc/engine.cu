@@ -615,26 +615,10 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     if (rc) return rc;
     // attention split scratch
     // sized for the decode step (one row per sequence)
-    // up to 1024 tokens of capacity the splits of a (row, KV head) are one cluster of at most 16 CTAs, one page
-    // per split while the context allows (a page is about 0.65 us of dependent instructions, so pages of a
-    // split cost more than the wider merge); longer caches need more CTAs than a cluster holds and merge
-    // through global scratch + ticket
-    // ... and only while the (row, KV head) pairs alone do not fill the GPU: with half an SM's worth of pairs or more
-    // the launch is a throughput problem (64 sequences stream 39 MB of pages per layer), which the cost model
-    // of attn_pick_nsplit answers with few splits of many pages each, i.e. the bulk-copy ring kernel
-    att_cluster_ = use_clusters_ && max_pages_ <= 64 && (long)batch * kvh_ < sm_count_ / 2;
-    // Decode passes of few (row, KV head) pairs stay clusters of sixteen CTAs on longer caches too (the streaming kernel from a few pages per CTA on, launch_tc): ms per
-    // step with splits through global scratch and so, 1.5 B with 1200 tokens 1.62 and 1.23, 2000 1.63 and 1.25 (bf16 pages 1.48 and 1.17), 4000 1.53 and
-    // 1.38; 0.5 B 1200 0.79 and 0.59, 4000 0.71 and 0.63; TinyLlama Q8_0 2000 0.76 and 0.67; two sequences of 1.5 B, 1500 1.70 and 1.29.  Eight pairs are 128 CTAs,
-    // which must share SMs to be eight clusters at once: f32 pages of 128-wide heads do not fit twice (0.6 B with 2000 0.76 and 0.79, 4000 0.81 and 0.96).
-    const long pairs = (long)batch * kvh_;
-    const int reach = pairs <= 4 ? 256 : pairs <= 8 ? (kv_bf16_ || hd_ == 64 ? 256 : 80) : 64;
-    att_decode_cluster_ = use_clusters_ && max_pages_ <= reach && pairs < sm_count_ / 2;
-    att_by_pages_ = attn_pick_cluster(max_pages_, std::min(max_cluster_, 16));
-    att_nsplit_ = att_cluster_ ? att_by_pages_ : std::max(att_decode_cluster_ ? att_by_pages_ : 1, attn_pick_nsplit(batch, kvh_, max_pages_, sm_count_, kv_bf16_));
+    att_plan_ = AttnPlan(batch, kvh_, hd_, kv_bf16_, max_pages_, sm_count_, use_clusters_, max_cluster_);
     if (!spec_.listed()) {
-        HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * hd_ * 4));
-        HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_nsplit_ * 2 * 4));
+        HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * hd_ * 4));
+        HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * 2 * 4));
         HM_CUDA(dev_alloc(&att_tickets_, (size_t)scratch_rows_ * kvh_ * 4));
         HM_CUDA(cudaMemset(att_tickets_, 0, (size_t)scratch_rows_ * kvh_ * 4));
     }
@@ -1129,19 +1113,11 @@ AttnArgs Engine::attn_args(int l, int M, const float* q, const int32_t* row_pos,
     at.heads = heads_;
     at.kv_heads = kvh_;
     at.hd = hd_;
-    // fewer splits when the rows alone fill the SMs: about two CTAs per SM on the cluster path (caches
-    // of up to 1024 tokens), the kernel's cost model on the long-context path
-    const bool decode = row_seq == nullptr, cluster = decode ? att_decode_cluster_ : att_cluster_;
-    at.nsplit = std::min(cluster ? att_by_pages_ : att_nsplit_, cluster ? std::min(std::max(1, (2 * sm_count_ + M * kvh_ - 1) / (M * kvh_)), 16) : attn_pick_nsplit(M, kvh_, max_pages_, sm_count_, kv_bf16_));
-    at.cluster = cluster ? 1 : 0;
+    const AttnCut cut = att_plan_.cut(M, row_seq == nullptr);
+    at.nsplit = cut.nsplit;
+    at.cluster = cut.cluster ? 1 : 0;
+    at.early_pages = cut.early_pages;
     at.stream_pages = 1;
-    // Decode passes: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs per SM may keep the pages
-    // of a split (eight at most) in slots of their own, which takes the loads in front of the wait; but shared memory keeps the next projection's CTAs, whose
-    // weights arrive meanwhile, off those SMs.  One page per split only where the launch is 32 CTAs or, with 128-wide heads, more than 64: ms per step with up
-    // to eight and so, one sequence, 1.5 B with 600 tokens 1.47 and 1.24, 0.5 B with 1000 0.66 and 0.56, 0.6 B with 1000 0.77 and 0.74; four sequences of 1000,
-    // 1.5 B 2.00 and 1.69; elsewhere the other way round, 0.5 B, four of 1000 (64-wide heads) 0.80 and 0.82, 1.5 B, two of 800 (64 CTAs) 1.36 and 1.43.
-    const long ctas = (long)M * kvh_ * at.nsplit;
-    at.early_pages = !decode ? 0 : ctas > 2L * sm_count_ ? 1 : ctas <= 32 || (hd_ == 128 && ctas > 64) ? 2 : 9;
     at.err_flag = err_flag_;
     at.scale = (float)(1.0 / std::sqrt((double)hd_));  // src/hf/emitter.rs:719
     at.out = attn_;

@@ -12,6 +12,7 @@
 
 #include "../../include/homura_b200.h"
 #include "common.cuh"
+#include "attn_plan.h"
 #include "attn_prefill.h"
 #include "gla.h"
 #include "gqa_attn.h"
@@ -356,10 +357,7 @@ class Engine {
     unsigned int* tickets_ = nullptr;
     float *att_acc_ = nullptr, *att_ml_ = nullptr;
     unsigned int* att_tickets_ = nullptr;
-    int att_nsplit_ = 1;
-    int att_by_pages_ = 1;  // splits of a cluster
-    bool att_cluster_ = true;
-    bool att_decode_cluster_ = true;  // of decode passes
+    AttnPlan att_plan_;
     int* err_flag_ = nullptr;
     unsigned int* fin_ticket_ = nullptr;  // ticket of the LM head's folded argmax
 

@@ -1,0 +1,53 @@
+"""How the attention launches of steps and small passes are cut (csrc/attn_plan.h), compiled for the host: what holds for every shape."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SOURCE = """
+#include "attn_plan.h"
+using namespace hm;
+extern "C" void cut(int batch, int kvh, int hd, int bf16, int pages, int clusters, int M, int decode, int* out) {
+    const AttnPlan p(batch, kvh, hd, bf16 != 0, pages, 148, clusters != 0, 16);
+    const AttnCut c = p.cut(M, decode != 0);
+    out[0] = c.nsplit; out[1] = c.cluster; out[2] = c.early_pages; out[3] = p.scratch_splits();
+    out[4] = attn_pick_nsplit(M, kvh, pages, 148, bf16 != 0); out[5] = attn_pick_nsplit(batch, kvh, pages, 148, bf16 != 0);
+}
+"""
+SHAPES = [(batch, kvh, hd, bf16, pages) for batch in (1, 2, 4, 8, 40) for kvh in (1, 2, 4, 8) for hd in (64, 128) for bf16 in (0, 1) for pages in (1, 2, 17, 64, 65, 80, 81, 100, 125, 157, 256, 257, 1000)]
+
+
+@pytest.fixture(scope="module")
+def cut(tmp_path_factory):
+    d = tmp_path_factory.mktemp("plan")
+    (d / "plan.cpp").write_text(SOURCE)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", os.path.join(ROOT, "homura_b200", "csrc"), "-o", str(d / "plan.so"), str(d / "plan.cpp")])
+    lib = C.CDLL(str(d / "plan.so"))
+
+    def call(shape, M, decode, clusters=True):
+        out = (C.c_int * 6)()
+        lib.cut(*shape, int(clusters), M, int(decode), out)
+        return dict(zip(("nsplit", "cluster", "early", "scratch", "model", "batch_model"), out))
+
+    return call
+
+
+def test_launches_fit_their_merge(cut):
+    for shape in SHAPES:
+        for clusters in (True, False):
+            for M, decode in ((shape[0], True), (1, False), (8, False), (40, False), (64, False)):
+                c = cut(shape, M, decode, clusters)
+                assert 1 <= c["nsplit"] <= (16 if c["cluster"] else c["scratch"]), (shape, M, decode, c)
+                assert (c["early"] > 0) == decode
+                assert clusters or not c["cluster"]
+
+
+def test_passes_over_several_rows_of_a_sequence_are_cut_as_without_clusters(cut):
+    """Beyond 1024 tokens only steps are clusters; the splits of the other passes know nothing of that."""
+    for shape in SHAPES:
+        if shape[-1] > 64:
+            for M in (1, 2, 8, 40, 64):
+                c = cut(shape, M, False)
+                assert not c["cluster"] and c["nsplit"] == min(c["model"], c["batch_model"]), (shape, M, c)
