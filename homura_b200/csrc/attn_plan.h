@@ -50,7 +50,7 @@ struct AttnCut {
 
 // What a cache's shape decides (made with the cache), and what a launch of M rows adds to it.
 struct AttnPlan {
-    int kvh = 1, hd = 64, max_pages = 1, sms = 148;
+    int kvh = 1, group = 1, hd = 64, max_pages = 1, sms = 148;
     bool bf16 = false;
     int by_pages = 1;             // splits of a cluster: a page each while the cache is short
     int batch_splits = 1;         // of a pass of as many rows as there are sequences through global scratch
@@ -58,7 +58,7 @@ struct AttnPlan {
     bool decode_cluster = false;  // steps: a row per sequence
 
     AttnPlan() = default;
-    AttnPlan(int batch, int kvh_, int hd_, bool bf16_, int pages, int sm_count, bool use_clusters, int max_cluster) : kvh(kvh_), hd(hd_), max_pages(pages), sms(sm_count), bf16(bf16_) {
+    AttnPlan(int batch, int heads, int kvh_, int hd_, bool bf16_, int pages, int sm_count, bool use_clusters, int max_cluster) : kvh(kvh_), group(heads / kvh_), hd(hd_), max_pages(pages), sms(sm_count), bf16(bf16_) {
         const long pairs = (long)batch * kvh;
         by_pages = std::max(1, std::min(pages, std::min(max_cluster, 16)));
         batch_splits = attn_pick_nsplit(batch, kvh, pages, sms, bf16);
@@ -81,6 +81,21 @@ struct AttnPlan {
     // Splits that the scratch of a row must hold: of every launch that goes through it.
     int scratch_splits() const { return cluster || decode_cluster ? std::max(by_pages, batch_splits) : batch_splits; }
 
+    // AttnArgs::early_pages of a decode pass: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs
+    // per SM may keep the pages of a split (eight at most) in slots of their own, which takes the loads in front of the wait; but shared memory keeps the next
+    // projection's CTAs, whose weights arrive meanwhile, off those SMs, and a page of 128-wide heads is 16 KB of it.  One slot per split and up to eight:
+    // - 64-wide heads: 0.5 B stack, one sequence, two pages per CTA 0.506 and 0.490 ms per step; four sequences of 1000 0.82 and 0.80.
+    // - 128-wide heads in clusters, launches of 32 CTAs: us per layer of eight heads and 300 tokens 22.2 and 23.4; of up to 64: 1.5 B, two sequences of 800
+    //   1.43 and 1.36 ms; of more: four of 1000 1.69 and 2.00 ms, but with two pages per CTA 35.3 and 33.5 us per layer of four of 300 (bf16 pages).
+    // - 128-wide heads through global scratch, us per layer: eight sequences of 1100 on two KV heads of eight 69 and 64, two of 1100 on eight of three 44 and 39;
+    //   where the CTA works on four pages at a time anyway (one or two heads per KV head) 36.8 and 39.2.
+    int early(long ctas, int pages_per_cta, bool in_cluster) const {
+        if (ctas > 2L * sms) return 1;
+        if (hd == 64) return 9;
+        if (!in_cluster) return group > 2 || ctas <= 64 ? 9 : 2;
+        return ctas <= 32 || (ctas > 64 && pages_per_cta > 2) ? 2 : 9;
+    }
+
     AttnCut cut(int M, bool decode) const {
         AttnCut c;
         c.cluster = decode ? decode_cluster : cluster;
@@ -88,13 +103,7 @@ struct AttnPlan {
         // that the rows of a prompt share their pages nor what the merge of so many partials costs: it is held to the splits of a step (a 40-row chunk
         // behind 1500 tokens of the 1.5 B shapes, bf16 pages: 77 us per layer with the step's 7 splits at most, 143 with the 16 of its clusters).
         c.nsplit = c.cluster ? std::min(by_pages, std::max(1, (2 * sms + M * kvh - 1) / (M * kvh))) : std::min(batch_splits, attn_pick_nsplit(M, kvh, max_pages, sms, bf16));
-        // Decode passes: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs per SM may keep the pages
-        // of a split (eight at most) in slots of their own, which takes the loads in front of the wait; but shared memory keeps the next projection's CTAs, whose
-        // weights arrive meanwhile, off those SMs.  One page per split only where the launch is 32 CTAs or, with 128-wide heads, more than 64: ms per step with up
-        // to eight and so, one sequence, 1.5 B with 600 tokens 1.47 and 1.24, 0.5 B with 1000 0.66 and 0.56, 0.6 B with 1000 0.77 and 0.74; four sequences of 1000,
-        // 1.5 B 2.00 and 1.69; elsewhere the other way round, 0.5 B, four of 1000 (64-wide heads) 0.80 and 0.82, 1.5 B, two of 800 (64 CTAs) 1.36 and 1.43.
-        const long ctas = (long)M * kvh * c.nsplit;
-        c.early_pages = !decode ? 0 : ctas > 2L * sms ? 1 : ctas <= 32 || (hd == 128 && ctas > 64) ? 2 : 9;
+        c.early_pages = !decode ? 0 : early((long)M * kvh * c.nsplit, (max_pages + c.nsplit - 1) / c.nsplit, c.cluster);
         return c;
     }
 };

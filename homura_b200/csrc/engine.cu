@@ -615,7 +615,7 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     if (rc) return rc;
     // attention split scratch
     // sized for the decode step (one row per sequence)
-    att_plan_ = AttnPlan(batch, kvh_, hd_, kv_bf16_, max_pages_, sm_count_, use_clusters_, max_cluster_);
+    att_plan_ = AttnPlan(batch, heads_, kvh_, hd_, kv_bf16_, max_pages_, sm_count_, use_clusters_, max_cluster_);
     if (!spec_.listed()) {
         HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * hd_ * 4));
         HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * 2 * 4));

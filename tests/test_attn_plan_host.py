@@ -9,14 +9,14 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SOURCE = """
 #include "attn_plan.h"
 using namespace hm;
-extern "C" void cut(int batch, int kvh, int hd, int bf16, int pages, int clusters, int M, int decode, int* out) {
-    const AttnPlan p(batch, kvh, hd, bf16 != 0, pages, 148, clusters != 0, 16);
+extern "C" void cut(int batch, int group, int kvh, int hd, int bf16, int pages, int clusters, int M, int decode, int* out) {
+    const AttnPlan p(batch, group * kvh, kvh, hd, bf16 != 0, pages, 148, clusters != 0, 16);
     const AttnCut c = p.cut(M, decode != 0);
     out[0] = c.nsplit; out[1] = c.cluster; out[2] = c.early_pages; out[3] = p.scratch_splits();
     out[4] = attn_pick_nsplit(M, kvh, pages, 148, bf16 != 0); out[5] = attn_pick_nsplit(batch, kvh, pages, 148, bf16 != 0);
 }
 """
-SHAPES = [(batch, kvh, hd, bf16, pages) for batch in (1, 2, 4, 8, 40) for kvh in (1, 2, 4, 8) for hd in (64, 128) for bf16 in (0, 1) for pages in (1, 2, 17, 64, 65, 80, 81, 100, 125, 157, 256, 257, 1000)]
+SHAPES = [(batch, group, kvh, hd, bf16, pages) for batch in (1, 2, 4, 8, 40) for group in (1, 3, 8) for kvh in (1, 2, 4, 8) for hd in (64, 128) for bf16 in (0, 1) for pages in (1, 2, 17, 64, 65, 80, 81, 100, 125, 157, 256, 257, 1000)]
 
 
 @pytest.fixture(scope="module")
@@ -51,3 +51,17 @@ def test_passes_over_several_rows_of_a_sequence_are_cut_as_without_clusters(cut)
             for M in (1, 2, 8, 40, 64):
                 c = cut(shape, M, False)
                 assert not c["cluster"] and c["nsplit"] == min(c["model"], c["batch_model"]), (shape, M, c)
+
+
+def test_pages_kept_in_shared_memory(cut):
+    """Through global scratch a split of 128-wide heads keeps its pages as long as two CTAs fit an SM, and splits of two pages keep them in clusters too."""
+    for shape in SHAPES:
+        batch, group, kvh, hd, _, pages = shape
+        c = cut(shape, batch, True)
+        ctas = batch * kvh * c["nsplit"]
+        if ctas > 2 * 148:
+            assert c["early"] == 1
+        elif hd == 64 or (not c["cluster"] and group > 2):
+            assert c["early"] == 9, (shape, c)
+        elif c["cluster"] and ctas > 32 and -(-pages // c["nsplit"]) == 2:
+            assert c["early"] == 9, (shape, c)
