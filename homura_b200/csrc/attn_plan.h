@@ -73,8 +73,10 @@ struct AttnPlan {
         // Decode passes of few (row, KV head) pairs stay clusters of sixteen CTAs on longer caches too (the streaming kernel from a few pages per CTA on, launch_tc): ms per
         // step with splits through global scratch and so, 1.5 B with 1200 tokens 1.62 and 1.23, 2000 1.63 and 1.25 (bf16 pages 1.48 and 1.17), 4000 1.53 and
         // 1.38; 0.5 B 1200 0.79 and 0.59, 4000 0.71 and 0.63; TinyLlama Q8_0 2000 0.76 and 0.67; two sequences of 1.5 B, 1500 1.70 and 1.29.  Eight pairs are 128 CTAs,
-        // which must share SMs to be eight clusters at once: f32 pages of 128-wide heads do not fit twice (0.6 B with 2000 0.76 and 0.79, 4000 0.81 and 0.96).
-        const int reach = pairs <= 4 ? 256 : pairs <= 8 ? (bf16 || hd == 64 ? 256 : 80) : 64;
+        // which must share SMs to be eight clusters at once: f32 pages of 128-wide heads do not fit twice (0.6 B with 1200 0.85 and 0.78, 2000 0.76 and 0.79, 4000 0.81 and
+        // 0.96).  On bf16 pages they do, but rank 0 of a cluster takes 16 results per query head and dimension: with six or eight heads of 128 per KV head
+        // longer caches are slower (1.5 B, four sequences of 4000 1.81 and 1.95 ms; us per layer at 2500 43.2 and 44.4, of eight heads, two sequences 42.3 and 40.6).
+        const int reach = pairs <= 4 ? 256 : pairs <= 8 ? (hd == 64 || (bf16 && group <= 4) ? 256 : bf16 ? 160 : 80) : 64;
         decode_cluster = use_clusters && pages <= reach && pairs < sms / 2;
     }
 

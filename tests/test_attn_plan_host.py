@@ -65,3 +65,9 @@ def test_pages_kept_in_shared_memory(cut):
             assert c["early"] == 9, (shape, c)
         elif c["cluster"] and ctas > 32 and -(-pages // c["nsplit"]) == 2:
             assert c["early"] == 9, (shape, c)
+
+
+def test_clusters_of_steps_on_long_caches(cut):
+    """Eight (row, KV head) pairs of many 128-wide heads leave the clusters beyond 2560 tokens; fewer pairs and fewer heads do not."""
+    for batch, group, kvh, hd, bf16, pages, want in [(4, 6, 2, 128, 1, 160, 1), (4, 6, 2, 128, 1, 161, 0), (2, 8, 4, 128, 1, 250, 0), (1, 2, 8, 128, 1, 250, 1), (4, 7, 2, 64, 0, 250, 1), (1, 8, 4, 128, 1, 250, 1), (1, 2, 8, 128, 0, 81, 0), (1, 2, 8, 128, 0, 80, 1)]:
+        assert cut((batch, group, kvh, hd, bf16, pages), batch, True)["cluster"] == want, (batch, group, kvh, hd, bf16, pages)
