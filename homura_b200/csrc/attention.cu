@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(ATT_THREADS, CL && HD == 128 ? 2 : 0) attn_dec
 // chunk-major K tile makes that read conflict-free while the query chunk is a broadcast), and a V row
 // is read once per token for g heads.  That cuts shared-memory traffic per page by about 3x against
 // one-warp-per-head, which is what bounds the kernel above on long contexts.  Used when a CTA has at
-// least ATT_ST_MIN_PAGES pages to read.
+// least ATT_ST_MIN_PAGES pages to read, in clusters from fewer on (attn_stream_from).
 constexpr int ST_THREADS = ATT_THREADS + 32;
 constexpr int ST_MAX_STAGES = 24;
 constexpr int ST_RING_BYTES = 64 * 1024;  // per CTA; two CTAs per SM keep 128 KB of pages in flight
@@ -1010,24 +1010,19 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     const long ctas = (long)a.nsplit * a.kv_heads * M;
     // A cluster's CTAs need as many SMs of one GPC at the same time: more than four clusters of sixteen want to share SMs.
     const bool crowd = CL && ctas > 64;
-    // Pages per CTA from which it streams.  In clusters it merges by asynchronous stores as well and soon wins: 1.5 B with 1000 tokens (four pages) 1.29 -> 1.22 ms
-    // per step, bf16 pages 1.30 -> 1.16; TinyLlama Q8_0 0.67 -> 0.65 and 0.61; two sequences of the 0.5 B stack with 900 0.66 -> 0.61.  One sequence on two
-    // 64-wide KV heads, 32 CTAs, from seven on (0.5 B: four pages 0.56 and 0.60, eight 0.65 and 0.63); CTAs that cannot share an SM from five on (0.6 B, f32
-    // pages: three 0.71 and 0.75, five 0.77 and 0.76; four sequences of 1.5 B on bf16 pages: four 1.71 and 1.77).
-    const int from = !CL ? ATT_ST_MIN_PAGES : HD == 64 && ctas <= 32 ? 7 : crowd && 2 * stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, StTile<HD, BF16>::STAGES) > 227 * 1024 ? 5 : 3;
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const bool two_fit = 2 * stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, StTile<HD, BF16>::STAGES) <= 227 * 1024;
+    const int from = CL ? attn_stream_from(HD, BF16, g, M, ctas, a.early_pages > 0, two_fit, sms) : ATT_ST_MIN_PAGES;
     const bool stream = a.stream_pages > 0 && pages_per_cta >= from && pages_per_cta <= ST_MAX_PT;
     // The ring bounds what one CTA keeps in flight (a warp asks for its next page only when it has freed a stage).
     // Launches that leave every CTA an SM to itself (64 sequences x 2 KV heads, one split: 128 CTAs) get as deep a
     // ring as shared memory holds, in multiples of the eight consumer warps; larger launches keep two CTAs per SM.
     using STT = StTile<HD, BF16>;
     int stages = STT::STAGES;
-    if (stream) {
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (ctas <= sms && !crowd) {
-            const int want = std::min(ST_MAX_STAGES, (pages_per_cta + ATT_WARPS - 1) / ATT_WARPS * ATT_WARPS);
-            while (stages + ATT_WARPS <= want && stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, stages + ATT_WARPS) <= 216 * 1024) stages += ATT_WARPS;
-        }
+    if (stream && ctas <= sms && !crowd) {
+        const int want = std::min(ST_MAX_STAGES, (pages_per_cta + ATT_WARPS - 1) / ATT_WARPS * ATT_WARPS);
+        while (stages + ATT_WARPS <= want && stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, stages + ATT_WARPS) <= 216 * 1024) stages += ATT_WARPS;
     }
     AttnArgs a2 = a;
     a2.st_stages = stages;

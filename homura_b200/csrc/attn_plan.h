@@ -4,7 +4,7 @@
 
 namespace hm {
 
-constexpr int ATT_ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used (in clusters: see launch_tc)
+constexpr int ATT_ST_MIN_PAGES = 16;  // pages per CTA from which the streaming variant is used (in clusters: attn_stream_from)
 
 // Splits per (row, KV head) through global scratch: minimise waves x (fixed cost per CTA + pages per CTA) + merge cost.
 // Units are "pages streamed by one CTA": the fixed cost (launch, query and page-table loads) is
@@ -39,6 +39,29 @@ inline int attn_pick_nsplit(int M, int kv_heads, int max_pages, int sm_count, bo
         }
     }
     return best;
+}
+
+// Pages per CTA from which the streaming kernel takes a launch in clusters: its warps take whole pages for all query heads, the short kernel's a head each.
+// two_fit: its shared memory leaves room for two CTAs per SM.  early: a row per sequence, pages are read ahead of the wait.  Short and streaming kernel:
+// - Up to a CTA per SM, from three pages on.  ms per step: 1.5 B with 1000 tokens (four pages) 1.29 and 1.22, bf16 pages 1.30 and 1.16; TinyLlama Q8_0 0.67 and 0.65;
+//   two sequences of the 0.5 B stack with 900 0.66 and 0.61; one of bf16 pages with 1000 0.56 and 0.535.  One sequence on f32 pages of more than four
+//   64-wide heads (32 CTAs) from five on: 0.5 B, four pages 0.555 and 0.563, five 0.583 and 0.572.  CTAs that cannot share an SM (f32 pages of 128-wide heads)
+//   from five on where there are more than 64: 0.6 B, three pages 0.71 and 0.75, five 0.77 and 0.76; four sequences of 1.5 B on bf16 pages, four 1.71 and 1.77.
+// - More CTAs than SMs, 64-wide heads, up to four rows: the next launch streams its weights into the shared memory that a ring would take.  us per layer, four
+//   sequences of 1000 on four KV heads of three 31.1 and 34.4 (f32 pages), of eight 37.6 and 43.0; seven pages 32.6 and 33.6.
+// - More, and more rows, steps: eight sequences, us per layer, four pages of one head 39.7 and 37.3, of eight 44.6 and 46.4, five of eight 49.0 and 47.8; bf16 pages,
+//   four of eight 45.4 and 43.6.
+// - More, rows that may not read ahead (prompt chunks, mixed batches): f32 pages, chunks of 40 rows on 128-wide heads, five pages 67.8 and 70.9, eight 77.9 and 74.4; on
+//   64-wide ones eight 64.0 and 65.0, thirteen 71.4 and 69.3; eight sequences, five 60.0 and 61.2, seven 64.4 and 62.7.  bf16 pages, 64-wide, chunks,
+//   four 55.6 and 59.1, five 59.1 and 58.9.
+inline int attn_stream_from(int hd, bool bf16, int group, int M, long ctas, bool early, bool two_fit, int sms) {
+    if (ctas > sms) {
+        if (hd == 64 && M <= 4) return ATT_ST_MIN_PAGES;
+        if (!bf16 && !early) return hd == 128 ? 8 : M <= 16 ? 7 : 10;
+        if (hd == 64) return early && (bf16 || group <= 2) ? 3 : 5;
+    }
+    if (hd == 64) return !bf16 && group > 4 && ctas <= 32 ? 5 : 3;
+    return ctas > 64 && !two_fit ? 5 : 3;
 }
 
 // One launch: splits of a (row, KV head), and whether they are a cluster.

@@ -16,6 +16,9 @@ extern "C" void cut(int batch, int group, int kvh, int hd, int bf16, int pages, 
     out[4] = attn_pick_nsplit(M, kvh, pages, 148, bf16 != 0); out[5] = attn_pick_nsplit(batch, kvh, pages, 148, bf16 != 0);
 }
 """
+SOURCE += '''
+extern "C" int stream_from(int hd, int bf16, int group, int M, int ctas, int early, int two_fit) { return attn_stream_from(hd, bf16 != 0, group, M, ctas, early != 0, two_fit != 0, 148); }
+'''
 SHAPES = [(batch, group, kvh, hd, bf16, pages) for batch in (1, 2, 4, 8, 40) for group in (1, 3, 8) for kvh in (1, 2, 4, 8) for hd in (64, 128) for bf16 in (0, 1) for pages in (1, 2, 17, 64, 65, 80, 81, 100, 125, 157, 256, 257, 1000)]
 
 
@@ -31,6 +34,7 @@ def cut(tmp_path_factory):
         lib.cut(*shape, int(clusters), M, int(decode), out)
         return dict(zip(("nsplit", "cluster", "early", "scratch", "model", "batch_model"), out))
 
+    call.lib = lib
     return call
 
 
@@ -71,3 +75,11 @@ def test_clusters_of_steps_on_long_caches(cut):
     """Eight (row, KV head) pairs of many 128-wide heads leave the clusters beyond 2560 tokens; fewer pairs and fewer heads do not."""
     for batch, group, kvh, hd, bf16, pages, want in [(4, 6, 2, 128, 1, 160, 1), (4, 6, 2, 128, 1, 161, 0), (2, 8, 4, 128, 1, 250, 0), (1, 2, 8, 128, 1, 250, 1), (4, 7, 2, 64, 0, 250, 1), (1, 8, 4, 128, 1, 250, 1), (1, 2, 8, 128, 0, 81, 0), (1, 2, 8, 128, 0, 80, 1)]:
         assert cut((batch, group, kvh, hd, bf16, pages), batch, True)["cluster"] == want, (batch, group, kvh, hd, bf16, pages)
+
+
+def test_pages_from_which_a_cluster_streams(cut):
+    """(head width, bf16 pages, heads per KV head, rows, CTAs, reads ahead, two CTAs per SM): pages.  Where the streaming kernel was the slower one it waits for more."""
+    for args, want in [((64, 0, 7, 1, 32, 1, 1), 5), ((64, 1, 7, 1, 32, 1, 1), 3), ((64, 0, 4, 1, 16, 1, 1), 3), ((64, 0, 8, 4, 128, 1, 1), 3), ((64, 0, 8, 4, 256, 1, 1), 16), ((64, 1, 1, 2, 256, 0, 1), 16),
+                       ((64, 0, 8, 8, 320, 1, 1), 5), ((64, 1, 8, 8, 256, 1, 1), 3), ((64, 0, 8, 8, 320, 0, 1), 7), ((64, 0, 7, 40, 320, 0, 1), 10), ((64, 1, 8, 40, 320, 0, 1), 5),
+                       ((128, 0, 6, 40, 320, 0, 0), 8), ((128, 1, 6, 40, 320, 0, 1), 3), ((128, 0, 2, 1, 128, 1, 0), 5), ((128, 0, 6, 1, 32, 1, 0), 3), ((128, 1, 6, 4, 128, 1, 0), 5)]:
+        assert cut.lib.stream_from(*args) == want, args
