@@ -347,10 +347,11 @@ __device__ __forceinline__ void merge_slots_and_write(const AttnArgs& a, int nsu
     if (tid == 0) a.tickets[m * a.kv_heads + kvh] = 0u;
 }
 
-// The cluster variants of 128-wide heads may take 128 registers: left to itself the compiler keeps them at 80 and spills, and a launch with a stack
-// costs the chain that it is part of 8 us (1.5 B, one sequence on bf16 pages: 1.54 -> 1.16 ms per step).
-template <int HD, bool BF16, bool CL>
-__global__ void __launch_bounds__(ATT_THREADS, CL && HD == 128 ? 2 : 0) attn_decode_kernel(const AttnArgs a) {
+// The cluster variants of 128-wide heads may take 128 registers.  On bf16 pages the compiler, left to itself, keeps to 80 and spills, and a launch with a stack costs the
+// chain that it is part of 8 us (1.5 B, one sequence: 1.54 -> 1.16 ms per step).  (On f32 pages it takes 84 and spills nothing; with 128 no step got slower.)
+// CROWD: 80 registers on bf16 pages all the same, where there are more CTAs than SMs and warps without a page (see launch_tc): a third CTA per SM counts for more.
+template <int HD, bool BF16, bool CL, bool CROWD = false>
+__global__ void __launch_bounds__(ATT_THREADS, CL && HD == 128 && !CROWD ? 2 : 0) attn_decode_kernel(const AttnArgs a) {
     using TL = Tile<HD, BF16>;
     using T = typename std::conditional<BF16, uint16_t, float>::type;
     constexpr int EPL = HD / 32;  // output elements per lane
@@ -1027,10 +1028,17 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     AttnArgs a2 = a;
     a2.st_stages = stages;
     const size_t smem = stream ? stream_smem_bytes<HD, BF16>(pages_per_cta, g, slots, stages) : smem_bytes<HD, BF16>(g, slots, pick_nslots<HD, BF16>(g, a.early_pages, a.max_pages, a.nsplit));
+    void (*kernel)(const AttnArgs) = attn_decode_kernel<HD, BF16, CL>;
+    if constexpr (CL && BF16 && HD == 128) {
+        // us per layer with 128 registers and with 80, three heads per KV head on eight: two sequences of 300 33.8 and 31.5, four 42.6 and 38.1; a mixed batch of eight
+        // of 800 with six heads on two 66.0 and 62.4.  Where all warps have a page (two heads per KV head) 31.7 and 32.7; steps of more than two pages per CTA, six heads 53.7 and 58.3.
+        if (ctas > sms && pick_nsub<HD, BF16>(g) * g < ATT_WARPS && (pages_per_cta <= 2 || a.early_pages == 0)) kernel = attn_decode_kernel<HD, BF16, CL, true>;
+    }
+    if (stream) kernel = attn_stream_kernel<HD, BF16, CL, GH>;
     // per device, and only ever raised: launches captured in a graph must stay valid after later calls
     {
-        cudaError_t e = stream ? ensure_dyn_smem(attn_stream_kernel<HD, BF16, CL, GH>, smem) : ensure_dyn_smem(attn_decode_kernel<HD, BF16, CL>, smem);
-        if (e == cudaSuccess && CL && a.nsplit > 8) e = stream ? ensure_nonportable_clusters(attn_stream_kernel<HD, BF16, CL, GH>) : ensure_nonportable_clusters(attn_decode_kernel<HD, BF16, CL>);
+        cudaError_t e = ensure_dyn_smem(kernel, smem);
+        if (e == cudaSuccess && CL && a.nsplit > 8) e = ensure_nonportable_clusters(kernel);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -1054,7 +1062,7 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
-    return stream ? cudaLaunchKernelEx(&cfg, attn_stream_kernel<HD, BF16, CL, GH>, a2) : cudaLaunchKernelEx(&cfg, attn_decode_kernel<HD, BF16, CL>, a2);
+    return cudaLaunchKernelEx(&cfg, kernel, a2);
 }
 
 template <int HD, bool BF16, bool CL>
