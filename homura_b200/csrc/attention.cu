@@ -638,8 +638,10 @@ __host__ __device__ constexpr size_t st_q_bytes(int hd) { return 3 * (size_t)(hd
 // GH: query heads per KV head on f32 pages.  The loops of a page are unrolled over the heads, and heads that may or may not be there cost a
 // test each, in loops that the issue rate bounds.  One variant for up to eight heads, and now: 8 sequences x 16384 tokens, 2 heads per KV head
 // of 128: 289 -> 173 us (6.2 TB/s); 6 heads of 128: 118 -> 78; 7 heads of 64: 51.7 -> 43.3; 64 x 500, 6 of 128: 34.7 -> 23.6.
+// Eight heads of 128 on f32 pages in clusters spilled at the 96 registers that two CTAs per SM leave, which 128 KB of ring do not allow anyway; with 158, us per layer: one sequence
+// on four KV heads with 2500 tokens 34.5 -> 30.9, on one with 800 25.1 -> 22.9, a 40-row chunk behind 1000 131 -> 112.
 template <int HD, bool BF16, bool CL, int GH>
-__global__ void __launch_bounds__(ST_THREADS, 2) attn_stream_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(ST_THREADS, CL && HD == 128 && !BF16 && GH == G_MAX ? 1 : 2) attn_stream_kernel(const AttnArgs a) {
     using ST = StTile<HD, BF16>;
     using T = typename std::conditional<BF16, uint16_t, float>::type;
     constexpr int EPL = HD / 32;

@@ -18,6 +18,8 @@ STACKS = {
     "6x128": dict(hidden_size=768, intermediate_size=512, num_attention_heads=6, num_key_value_heads=1, head_dim=128),
     "2x128": dict(hidden_size=256, intermediate_size=256, num_attention_heads=16, num_key_value_heads=8, head_dim=128, qkv_bias=False, qk_norm=True),
     "3x128": dict(hidden_size=256, intermediate_size=256, num_attention_heads=24, num_key_value_heads=8, head_dim=128),
+    "8x128": dict(hidden_size=256, intermediate_size=256, num_attention_heads=32, num_key_value_heads=4, head_dim=128),
+    "8x64": dict(hidden_size=256, intermediate_size=256, num_attention_heads=32, num_key_value_heads=4, head_dim=64),
 }
 _made = {}
 
@@ -36,6 +38,7 @@ CASES = [
     ("6x128", 1, 500, 479, "f32"), ("6x128", 2, 1000, 40, "bf16"), ("6x128", 4, 2100, 700, "f32"), ("6x128", 8, 1040, 50, "f32"),
     ("2x128", 1, 700, 681, "f32"), ("2x128", 1, 1000, 975, "bf16"), ("2x128", 1, 1200, 1180, "f32"), ("2x128", 1, 1300, 630, "f32"), ("2x128", 1, 2000, 1100, "bf16"), ("2x128", 2, 1010, 64, "f32"),
     ("3x128", 2, 300, 281, "bf16"), ("3x128", 4, 500, 300, "bf16"), ("3x128", 8, 120, 101, "bf16"), ("3x128", 2, 700, 60, "bf16"),
+    ("8x128", 1, 700, 679, "f32"), ("8x128", 1, 4100, 2050, "f32"), ("8x128", 2, 1200, 1190, "f32"), ("8x128", 1, 2560, 1295, "bf16"), ("8x64", 1, 800, 790, "f32"), ("8x64", 1, 4096, 1500, "bf16"), ("8x64", 4, 900, 880, "f32"),
 ]
 
 
