@@ -109,14 +109,14 @@ struct AttnPlan {
     // AttnArgs::early_pages of a decode pass: one row per sequence (prefill chunks write several positions of one sequence).  Launches of at most two CTAs
     // per SM may keep the pages of a split (eight at most) in slots of their own, which takes the loads in front of the wait; but shared memory keeps the next
     // projection's CTAs, whose weights arrive meanwhile, off those SMs, and a page of 128-wide heads is 16 KB of it.  One slot per split and up to eight:
-    // - 64-wide heads: 0.5 B stack, one sequence, two pages per CTA 0.506 and 0.490 ms per step; four sequences of 1000 0.82 and 0.80.
+    // - 64-wide heads: 0.5 B stack, one sequence, two pages per CTA 0.506 and 0.490 ms per step, four of them (32 CTAs) 0.555 and 0.576; four sequences of 1000 0.82 and 0.80.
     // - 128-wide heads in clusters, launches of 32 CTAs: us per layer of eight heads and 300 tokens 22.2 and 23.4; of up to 64: 1.5 B, two sequences of 800
     //   1.43 and 1.36 ms; of more: four of 1000 1.69 and 2.00 ms, but with two pages per CTA 35.3 and 33.5 us per layer of four of 300 (bf16 pages).
     // - 128-wide heads through global scratch, us per layer: eight sequences of 1100 on two KV heads of eight 69 and 64, two of 1100 on eight of three 44 and 39;
     //   where the CTA works on four pages at a time anyway (one or two heads per KV head) 36.8 and 39.2.
     int early(long ctas, int pages_per_cta, bool in_cluster) const {
         if (ctas > 2L * sms) return 1;
-        if (hd == 64) return 9;
+        if (hd == 64) return in_cluster && ctas <= 32 && pages_per_cta > 2 ? 2 : 9;
         if (!in_cluster) return group > 2 || ctas <= 64 ? 9 : 2;
         return ctas <= 32 || (ctas > 64 && pages_per_cta > 2) ? 2 : 9;
     }
