@@ -1025,7 +1025,7 @@ size_t smem_bytes(int g, int slots, int nslots) {
 }
 
 template <int HD, bool BF16, bool CL, int GH>
-cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
+cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl, int* clusters) {
     const int g = a.heads / a.kv_heads;
     const int pages_per_cta = (a.max_pages + a.nsplit - 1) / a.nsplit;
     // long contexts: the bulk-copy ring; a slot layout needs ATT_WARPS / g >= 1 as in the kernel above
@@ -1084,41 +1084,42 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
     }
     cfg.attrs = at;
     cfg.numAttrs = n;
+    if (clusters) return CL ? cudaOccupancyMaxActiveClusters(clusters, kernel, &cfg) : cudaErrorInvalidValue;
     return cudaLaunchKernelEx(&cfg, kernel, a2);
 }
 
 template <int HD, bool BF16, bool CL>
-cudaError_t launch_g(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
+cudaError_t launch_g(const AttnArgs& a, int M, cudaStream_t st, bool pdl, int* clusters) {
     const int g = a.heads / a.kv_heads;
     if constexpr (!BF16) {
         switch (g) {
-            case 1: return launch_tc<HD, BF16, CL, 1>(a, M, st, pdl);
-            case 2: return launch_tc<HD, BF16, CL, 2>(a, M, st, pdl);
-            case 3: return launch_tc<HD, BF16, CL, 3>(a, M, st, pdl);
-            case 4: return launch_tc<HD, BF16, CL, 4>(a, M, st, pdl);
-            case 5: return launch_tc<HD, BF16, CL, 5>(a, M, st, pdl);
-            case 6: return launch_tc<HD, BF16, CL, 6>(a, M, st, pdl);
-            case 7: return launch_tc<HD, BF16, CL, 7>(a, M, st, pdl);
+            case 1: return launch_tc<HD, BF16, CL, 1>(a, M, st, pdl, clusters);
+            case 2: return launch_tc<HD, BF16, CL, 2>(a, M, st, pdl, clusters);
+            case 3: return launch_tc<HD, BF16, CL, 3>(a, M, st, pdl, clusters);
+            case 4: return launch_tc<HD, BF16, CL, 4>(a, M, st, pdl, clusters);
+            case 5: return launch_tc<HD, BF16, CL, 5>(a, M, st, pdl, clusters);
+            case 6: return launch_tc<HD, BF16, CL, 6>(a, M, st, pdl, clusters);
+            case 7: return launch_tc<HD, BF16, CL, 7>(a, M, st, pdl, clusters);
         }
     }
-    return launch_tc<HD, BF16, CL, G_MAX>(a, M, st, pdl);
+    return launch_tc<HD, BF16, CL, G_MAX>(a, M, st, pdl, clusters);
 }
 
 template <int HD, bool BF16>
-cudaError_t launch_t(const AttnArgs& a, int M, cudaStream_t st, bool pdl) {
+cudaError_t launch_t(const AttnArgs& a, int M, cudaStream_t st, bool pdl, int* clusters) {
     if (a.cluster) {
         if (a.nsplit < 1 || a.nsplit > 16) return cudaErrorInvalidValue;
-        return launch_g<HD, BF16, true>(a, M, st, pdl);
+        return launch_g<HD, BF16, true>(a, M, st, pdl, clusters);
     }
-    return launch_g<HD, BF16, false>(a, M, st, pdl);
+    return launch_g<HD, BF16, false>(a, M, st, pdl, clusters);
 }
 
 }  // namespace
 
-cudaError_t launch_attn_decode(const AttnArgs& a, int M, bool kv_bf16, cudaStream_t st, bool pdl) {
+cudaError_t launch_attn_decode(const AttnArgs& a, int M, bool kv_bf16, cudaStream_t st, bool pdl, int* clusters) {
     if (a.page_tokens != PT || a.heads % a.kv_heads != 0 || a.heads / a.kv_heads > G_MAX) return cudaErrorInvalidValue;
-    if (a.hd == 64) return kv_bf16 ? launch_t<64, true>(a, M, st, pdl) : launch_t<64, false>(a, M, st, pdl);
-    if (a.hd == 128) return kv_bf16 ? launch_t<128, true>(a, M, st, pdl) : launch_t<128, false>(a, M, st, pdl);
+    if (a.hd == 64) return kv_bf16 ? launch_t<64, true>(a, M, st, pdl, clusters) : launch_t<64, false>(a, M, st, pdl, clusters);
+    if (a.hd == 128) return kv_bf16 ? launch_t<128, true>(a, M, st, pdl, clusters) : launch_t<128, false>(a, M, st, pdl, clusters);
     return cudaErrorInvalidValue;
 }
 

@@ -133,4 +133,15 @@ struct AttnPlan {
     }
 };
 
+// A cluster wants that many SMs of one GPC at once, with the shared memory of its CTAs free: where the device has no room for a launch that a plan holds (fits) its
+// clusters are eight CTAs, and there are none where these do not fit either.
+template <class Fits>
+AttnPlan attn_plan_that_fits(int batch, int heads, int kvh, int hd, bool bf16, int pages, int sm_count, bool use_clusters, int max_cluster, Fits fits) {
+    for (int most : {max_cluster, 8}) {
+        const AttnPlan p(batch, heads, kvh, hd, bf16, pages, sm_count, use_clusters, most);
+        if ((!p.cluster && !p.decode_cluster) || fits(p)) return p;
+    }
+    return AttnPlan(batch, heads, kvh, hd, bf16, pages, sm_count, false, 8);
+}
+
 }  // namespace hm

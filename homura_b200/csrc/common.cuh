@@ -555,7 +555,8 @@ void gemv_pick_split(int K, int N, int M, int sm_count, int* ksplit, int* rows_p
 // Cluster variant: ksplit = cluster size (<= max_cluster), sized so that all CTAs are resident at once.
 void gemv_pick_cluster(int K, int N, int M, int sm_count, int max_cluster, int* cluster, int* rows_per_split);
 int gemv_max_cluster();  // largest cluster size the device schedules for the projection kernel (8 or 16)
-cudaError_t launch_attn_decode(const AttnArgs& a, int M, bool kv_bf16, cudaStream_t st, bool pdl);
+// clusters: launches nothing and says how many of the launch's clusters the device holds at once
+cudaError_t launch_attn_decode(const AttnArgs& a, int M, bool kv_bf16, cudaStream_t st, bool pdl, int* clusters = nullptr);
 
 // k_total > 0: the rows are inputs [k_off, k_off + K) of a projection over k_total inputs
 cudaError_t launch_pack_slabs_from_nk(const uint16_t* src_nk, int N, int K, uint16_t* dst, int n_off, int interleave_which, cudaStream_t st, int k_total = 0, int k_off = 0);

@@ -615,7 +615,7 @@ int Engine::kv_alloc(int batch, int max_seq_len, int page_tokens, int kv_dtype, 
     if (rc) return rc;
     // attention split scratch
     // sized for the decode step (one row per sequence)
-    att_plan_ = AttnPlan(batch, heads_, kvh_, hd_, kv_bf16_, max_pages_, sm_count_, use_clusters_, max_cluster_);
+    att_plan_ = attn_plan_that_fits(batch, heads_, kvh_, hd_, kv_bf16_, max_pages_, sm_count_, use_clusters_ && !spec_.listed(), max_cluster_, [this](const AttnPlan& p) { return clusters_fit(p); });
     if (!spec_.listed()) {
         HM_CUDA(dev_alloc(&att_acc_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * hd_ * 4));
         HM_CUDA(dev_alloc(&att_ml_, (size_t)scratch_rows_ * heads_ * att_plan_.scratch_splits() * 2 * 4));
@@ -1097,6 +1097,21 @@ int Engine::enqueue_linear(const LinearW& L, int M, const float* x, int ldx, int
     pf_ptr_ = nullptr;
     pf_bytes_ = 0;
     return HM_OK;
+}
+
+// Steps, and passes over several rows of a sequence of every size.
+bool Engine::clusters_fit(const AttnPlan& plan) {
+    att_plan_ = plan;
+    auto fits = [&](int M, const int32_t* row_seq) {
+        const AttnArgs at = attn_args(0, M, q_, pos_dev_, row_seq);
+        int n = 0;
+        if (!at.cluster || launch_attn_decode(at, M, kv_bf16_, stream_, false, &n) == cudaSuccess) return !at.cluster || n > 0;
+        cudaGetLastError();
+        return false;
+    };
+    bool all = fits(batch_, nullptr);
+    for (int M = 1; all && M <= scratch_rows_; ++M) all = fits(M, seq_iota_);
+    return all;
 }
 
 AttnArgs Engine::attn_args(int l, int M, const float* q, const int32_t* row_pos, const int32_t* row_seq) const {

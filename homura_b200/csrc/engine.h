@@ -358,6 +358,7 @@ class Engine {
     float *att_acc_ = nullptr, *att_ml_ = nullptr;
     unsigned int* att_tickets_ = nullptr;
     AttnPlan att_plan_;
+    bool clusters_fit(const AttnPlan& plan);  // on this device, with the shared memory of the launches
     int* err_flag_ = nullptr;
     unsigned int* fin_ticket_ = nullptr;  // ticket of the LM head's folded argmax
 
