@@ -1185,14 +1185,15 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
     // Weight prefetch, decode passes of bf16 models: every kernel asks the L2 for the weights of the
     // kernel two launches ahead, so HBM keeps streaming while the short dependent kernels run.
     const bool pf = use_prefetch_ && !quant_ && !tall && only_class_ < 0;
-    auto prefetch = [&](const LinearW* w, size_t off = 0, size_t cap = ~(size_t)0) {
+    auto prefetch = [&](const LinearW* w, size_t off = 0) {
         pf_ptr_ = nullptr;
         pf_bytes_ = 0;
         if (!pf || !w || !w->slabs || off >= w->bytes()) return;
         pf_ptr_ = (const char*)w->slabs + off;
-        pf_bytes_ = std::min(cap, std::min(PROJ_PF, w->bytes() - off));
+        pf_bytes_ = std::min(PROJ_PF, w->bytes() - off);
     };
-    constexpr size_t LM_PF = 24u << 20;  // the LM head does not fit the L2: only its first 2 x 24 MB are fetched early
+    // The LM head does not fit the L2: the last two projections ask for its first 8 MB and for the next.  (Two times 24 MB: 0.5 B 0.477 and 0.474 ms per step, 1.5 B 1.023
+    // and 1.019, with 1000 tokens 1.059 and 1.056; a hole of 16 MB between the two: no difference.)
     int rc;
     // passes of 5..64 rows: the attention output and the SwiGLU output go straight into the packed
     // activation tiles of the next tensor-core GEMM (no packing launch in between) ...
@@ -1275,7 +1276,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
             if (rc) return rc;
         } else if (w.gu.kind == HM_BF16) {
             if (l + 1 < L_) prefetch(&layers_[l + 1].qkv);
-            else if (lm_rows > 0) prefetch(&lm_head_, 0, LM_PF);
+            else if (lm_rows > 0) prefetch(&lm_head_);
             rc = enqueue_linear(w.gu, M, h_, H_, PRO_RMSNORM, w.post_ln, EPI_SWIGLU, act_, I_, nullptr, nullptr, l, row_pos, row_seq, nullptr, nullptr, launches);
             if (rc) return rc;
         } else {
@@ -1293,7 +1294,7 @@ int Engine::enqueue_pass(int M, const uint32_t* tokens_dev, const int32_t* row_p
             rc = enqueue_linear_tc(w.down, M, act_, I_, nullptr, EPI_STORE, h_, H_, nullptr, h_, l, row_pos, row_seq, launches, direct_pack ? xpack_act_ : nullptr, nullptr, fused ? &f : nullptr);
             if (rc) return rc;
         } else if (want(PC_DOWN)) {
-            if (l + 1 == L_ && lm_rows > 0) prefetch(&lm_head_, LM_PF, LM_PF);
+            if (l + 1 == L_ && lm_rows > 0) prefetch(&lm_head_, PROJ_PF);
             rc = enqueue_linear(w.down, M, act_, I_, PRO_PLAIN, nullptr, EPI_STORE, h_, H_, nullptr, h_, l, row_pos, row_seq, nullptr, nullptr, launches);
             if (rc) return rc;
         }
