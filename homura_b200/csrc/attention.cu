@@ -612,7 +612,7 @@ __device__ __forceinline__ float4 ld_chunk4(const void* tile, int elem) {  // 4 
 //   out^T    [hd x 8 heads]        += V^T    [hd x 16 tokens]   . P^T [16 tokens x 8 heads]
 // K and V are bf16 already; the f32 operands (Q, P) are split into three bf16 terms each (hi + mid + lo is
 // exact to 2^-24), one MMA per term, so the products are the f32 x bf16 products of the reference and only
-// the order of the f32 accumulation differs.  (The 8 heads of the MMA's N are the <= 8 query heads of the
+// the accumulation differs.  (The 8 heads of the MMA's N are the <= 8 query heads of the
 // KV head: the floordiv head map again.)
 __device__ __forceinline__ void mma_bf16_m16n8k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -640,7 +640,8 @@ __host__ __device__ constexpr size_t st_q_bytes(int hd) { return 3 * (size_t)(hd
 // of 128: 289 -> 173 us (6.2 TB/s); 6 heads of 128: 118 -> 78; 7 heads of 64: 51.7 -> 43.3; 64 x 500, 6 of 128: 34.7 -> 23.6.
 // Eight heads of 128 on f32 pages in clusters spilled at the 96 registers that two CTAs per SM leave, which 128 KB of ring do not allow anyway; with 158, us per layer: one sequence
 // on four KV heads with 2500 tokens 34.5 -> 30.9, on one with 800 25.1 -> 22.9, a 40-row chunk behind 1000 131 -> 112.
-template <int HD, bool BF16, bool CL, int GH>
+// STEP: steps in clusters on bf16 pages, which the kernel above took before: as accurate as there (scores^T below).  All other launches keep their sums as they are.
+template <int HD, bool BF16, bool CL, int GH, bool STEP = false>
 __global__ void __launch_bounds__(ST_THREADS, CL && HD == 128 && !BF16 && GH == G_MAX ? 1 : 2) attn_stream_kernel(const AttnArgs a) {
     using ST = StTile<HD, BF16>;
     using T = typename std::conditional<BF16, uint16_t, float>::type;
@@ -794,17 +795,26 @@ __global__ void __launch_bounds__(ST_THREADS, CL && HD == 128 && !BF16 && GH == 
                 const unsigned char* vt = ring + (size_t)s * ST::STAGE_BYTES + ST::TILE_BYTES;
                 const int p = p0 + i;
                 // ---- scores^T = K tile . Q^T ----
-                float sc[4] = {0.f, 0.f, 0.f, 0.f};
+                // The tensor core cuts off what it adds to a sum.  STEP: the leading terms go to two sums of half the length, the small ones to a third, and the three meet in
+                // f32.  Error of the logits of a step with 1000 tokens against 64 bits, rms, all in one chain, with f32 FMAs (the kernel above) and so: eight heads of two
+                // with QK-norm 1.93e-7, 0.93e-7 and 0.86e-7, six of 128 0.86e-7, 0.76e-7 and 0.64e-7; times are the same.  (A page's P . V in sums of its own
+                // as well spills 8 bytes on 128-wide heads: 1.5 B with 1000 tokens 1.061 and 1.075 ms per step.)
+                float sc[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int kt = 0; kt < HD / 16; ++kt) {
                     // chunk-major K tile: element (token, dim) at ((dim / 4) * 16 + token) * 4 + dim % 4
                     const int w0 = ((kt * 4 + (tig >> 1)) * 16 + gid) * 2 + (tig & 1);
                     const uint32_t a0 = kt32[w0], a1 = kt32[w0 + 16], a2 = kt32[w0 + 64], a3 = kt32[w0 + 80];
 #pragma unroll
-                    for (int t3 = 0; t3 < 3; ++t3) {
+                    for (int n3 = 0; n3 < 3; ++n3) {
+                        const int t3 = STEP ? 2 - n3 : n3;
                         const uint2 b = qf[(t3 * (HD / 16) + kt) * 32 + lane];
-                        mma_bf16_m16n8k16(sc, a0, a1, a2, a3, b.x, b.y);
+                        mma_bf16_m16n8k16(!STEP ? sc : t3 ? low : kt & 1 ? odd : sc, a0, a1, a2, a3, b.x, b.y);
                     }
+                }
+                if constexpr (STEP) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) sc[c] = (sc[c] + odd[c]) + low[c];
                 }
                 // An infinite key times a query term of zero, or times two terms of unlike signs, is not a number where key times query is an infinity (a weight
                 // of zero if it is the lower one): such scores are summed again in f32, as the kernel above does.
@@ -872,7 +882,7 @@ __global__ void __launch_bounds__(ST_THREADS, CL && HD == 128 && !BF16 && GH == 
                     uint32_t av[4];
                     ldmatrix_x4_trans(av, vrow + (size_t)mt * (2 * PT * 8 * 2));
 #pragma unroll
-                    for (int t3 = 0; t3 < 3; ++t3) mma_bf16_m16n8k16(to[mt], av[0], av[1], av[2], av[3], b0[t3], b1[t3]);
+                    for (int n3 = 0; n3 < 3; ++n3) mma_bf16_m16n8k16(to[mt], av[0], av[1], av[2], av[3], b0[STEP ? 2 - n3 : n3], b1[STEP ? 2 - n3 : n3]);
                 }
                 __syncwarp();
                 if (lane == 0) mb_arrive(&empty[s]);  // the stage may be refilled
@@ -1057,6 +1067,9 @@ cudaError_t launch_tc(const AttnArgs& a, int M, cudaStream_t st, bool pdl, int* 
         if (ctas > sms && pick_nsub<HD, BF16>(g) * g < ATT_WARPS && (pages_per_cta <= 2 || a.early_pages == 0)) kernel = attn_decode_kernel<HD, BF16, CL, true>;
     }
     if (stream) kernel = attn_stream_kernel<HD, BF16, CL, GH>;
+    if constexpr (CL && BF16) {
+        if (stream && a.early_pages > 0) kernel = attn_stream_kernel<HD, BF16, CL, GH, true>;
+    }
     // per device, and only ever raised: launches captured in a graph must stay valid after later calls
     {
         cudaError_t e = ensure_dyn_smem(kernel, smem);

@@ -122,3 +122,26 @@ def test_a_key_that_is_an_infinity_takes_its_row_out(hm, stack, cap, n, pages):
     want = step.logits(keys, values)
     assert np.isfinite(want).all()
     assert np.abs(_run(hm, d, cap, pages, token, keys, values) - want).max() <= 1e-4 * max(1.0, float(np.abs(want).max()))
+
+
+@pytest.mark.parametrize("stack", sorted(STACKS))
+def test_a_larger_cache_is_no_less_accurate(hm, stack):
+    """The same rows on bf16 pages in a cache whose steps run the short kernel (two pages per CTA, f32 FMAs) and in one whose steps stream (four; tensor cores):
+    medians over 24 tokens of the rms error of 512 logits scatter by a few percent, a bit less of precision doubles them."""
+    cfg, d, w = _stack(stack)
+    n = 490
+    keys, values = _rows(cfg, n)
+    want = [Step(cfg, w, token, n, "bf16").logits(keys, values) for token in range(24)]
+    errors = []
+    for cap in (512, 1000):
+        m = hm.HfModel.load_with_dtype(d, hm.DType.BF16)
+        m.init_kv_cache(cap, kv_dtype=hm.DType.BF16)
+        rms = []
+        for token in range(24):
+            m.reset_kv_cache()
+            m.kv_append(0, keys[None], values[None], advance=True)
+            got, _ = m.decode_step([token])
+            rms.append(float(np.sqrt(((got[0] - want[token]) ** 2).mean())))
+        m.close()
+        errors.append(float(np.median(rms)))
+    assert errors[1] <= 1.25 * errors[0], errors
