@@ -1,7 +1,7 @@
-"""Decode steps over caches of every size that changes how the attention of a step is launched: splits without a page (which only ask for weights), pages
+"""Decode steps over caches of every size that changes how the attention of a step is launched: splits without a page, pages
 kept in shared memory, streaming clusters, caches of more than 1024 tokens; logits of every step against the CPU oracle.
 
-Tolerance on f32 pages: that of the model tests, 1e-4 of the largest logit.  On bf16 pages 2e-2: keys and values that lie between two bf16 values go to the
+Tolerance on f32 pages: that of the model tests, 1e-4 of the largest logit (of one where that is less).  On bf16 pages 2e-2: keys and values that lie between two bf16 values go to the
 one or the other with the last bit of an f32 sum, 2^-8 of a value each."""
 import tempfile
 
